@@ -18,10 +18,11 @@
 // seed pool sorted by the GNU introsort (kgraph.cpp:476), neighbours visited
 // in adjacency order S at a time, each inserted with UpdateKnnList
 // semantics, k reset to the insert position (kgraph.cpp:478-514).  The
-// distances of one batch of S neighbours are computed in parallel (they are
-// pure), then inserted one by one in order, which is what the reference's
-// interleaved loop produces.  With the canonical distance this reproduces
-// the reference's ids, distances, result count and SearchInfo.cost exactly.
+// distances of a run of neighbours -- of several batches of S -- are computed
+// in parallel (they are pure), then merged up to the batch after which the
+// reference turns to another entry, which is what its interleaved loop
+// produces.  With the canonical distance this reproduces the reference's ids,
+// distances, result count and SearchInfo.cost exactly.
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
 #include <algorithm>
@@ -56,10 +57,14 @@ struct WarpSmem {
     uint32_t *pm;      // cap   m | (M << 16)
     float *rd;         // rcap  (T > 1 result merge)
     uint32_t *rid;     // rcap
-    float *cd;         // 32    batch distances
+    float *cd;         // 32    batch distances (seeds, brute force)
     uint32_t *cid;     // 32    batch ids
-    uint32_t *cM;      // 32    batch actual_M
+    // the walk's use of the same 96 words: a window's unvisited neighbours in order
+    uint32_t *lid;     // 64    ids
+    uint8_t *lpos;     // 64    positions in the window
+    uint8_t *lsel;     // 32    group lanes the compressed-row filter kept
 };
+constexpr uint32_t LIST = 64;   // entries of lid / lpos
 
 template <int CP>
 __device__ __forceinline__ WarpSmem carve(char *base, const SearchArgs &a) {
@@ -72,9 +77,11 @@ __device__ __forceinline__ WarpSmem carve(char *base, const SearchArgs &a) {
     if constexpr (!CP) { s.pm = reinterpret_cast<uint32_t *>(p); p += sizeof(uint32_t) * a.cap; }
     s.rd = reinterpret_cast<float *>(p); p += sizeof(float) * a.rcap;
     s.rid = reinterpret_cast<uint32_t *>(p); p += sizeof(uint32_t) * a.rcap;
-    s.cd = reinterpret_cast<float *>(p); p += sizeof(float) * 32;
-    s.cid = reinterpret_cast<uint32_t *>(p); p += sizeof(uint32_t) * 32;
-    s.cM = reinterpret_cast<uint32_t *>(p);
+    s.cd = reinterpret_cast<float *>(p);
+    s.cid = reinterpret_cast<uint32_t *>(p + sizeof(float) * 32);
+    s.lid = reinterpret_cast<uint32_t *>(p); p += sizeof(uint32_t) * LIST;
+    s.lpos = reinterpret_cast<uint8_t *>(p); p += LIST;
+    s.lsel = reinterpret_cast<uint8_t *>(p);
     return s;
 }
 
@@ -136,27 +143,21 @@ __device__ uint32_t warp_bruteforce(const SearchArgs &a, const WarpSmem &s, floa
     return L;
 }
 
-// Distances of the candidate lanes in `cm` (each holds its id), computed 32/G
-// at a time by the G-lane groups; every candidate lane returns its own distance.
-// The candidates' ids are compacted through the warp's 32-entry staging array
-// (rank order), the distances come back by shuffle.
+// Distances of the n <= 32 candidates list[0 .. n), computed 32/G at a time by
+// the G-lane groups; lane i < n returns candidate i's.  With `sel`, candidate i
+// is list[sel[i]].
 template <int G>
-__device__ __forceinline__ float warp_cand_dist(const SearchArgs &a, const float *q, float qn, uint32_t *stage,
-                                               unsigned cm, bool cand, uint32_t id, int lane) {
+__device__ __forceinline__ float warp_list_dist(const SearchArgs &a, const float *q, float qn, const uint32_t *list,
+                                               const uint8_t *sel, uint32_t n, int lane) {
     constexpr uint32_t PER = 32 / G;
     const int g = lane / G, t = lane % G;
-    const uint32_t n = __popc(cm);
-    const uint32_t my = __popc(cm & ((1u << lane) - 1u));
     float mine = 0.f;
-    if (cand) stage[my] = id;
-    __syncwarp();
     for (uint32_t base = 0; base < n; base += PER) {
         const uint32_t i = base + g;
-        const float dd = query_dist_g<G>(a.D, q, qn, i < n ? stage[i] : 0u, t, FULL);
-        const float got = __shfl_sync(FULL, dd, (int)(G * (my % PER)));
-        if (cand && my / PER == base / PER) mine = got;
+        const float dd = query_dist_g<G>(a.D, q, qn, i < n ? list[sel ? sel[i] : i] : 0u, t, FULL);
+        const float got = __shfl_sync(FULL, dd, (int)(G * (lane % PER)));
+        if ((uint32_t)lane / PER == base / PER) mine = got;
     }
-    __syncwarp();   // the staging array is reused by the next batch
     return mine;
 }
 
@@ -268,26 +269,22 @@ __device__ __forceinline__ float filter_lb(int metric, float raw, float e, float
     return __fsub_rd(__fmul_rd(t2, 0.5f), __fmul_ru(2.2f * gc, __fadd_ru(nq, nx)));
 }
 
-// Lower bounds of the candidate lanes in `cm` from their compressed rows,
-// 32/G per pass; every candidate lane returns its own bound.
+// Lower bounds of the n <= 32 candidates list[0 .. n) from their compressed
+// rows, 32/G per pass; lane i < n returns candidate i's.
 template <int PREC, int G>
-__device__ __forceinline__ float warp_cand_lb(const SearchArgs &a, const float *q, float qn, unsigned cm, bool cand,
-                                              uint32_t id, int lane) {
+__device__ __forceinline__ float warp_list_lb(const SearchArgs &a, const float *q, float qn, const uint32_t *list,
+                                              uint32_t n, int lane) {
     constexpr uint32_t PER = 32 / G;
     const int g = lane / G, t = lane % G;
-    const uint32_t n = __popc(cm);
-    const uint32_t my = __popc(cm & ((1u << lane) - 1u));
     float mine = 0.f;
     for (uint32_t base = 0; base < n; base += PER) {
         const uint32_t i = base + g;
-        const int src = i < n ? (int)__fns(cm, 0, i + 1) : 0;
-        const uint32_t cid = __shfl_sync(FULL, id, src);
-        const uint32_t row = i < n ? cid : 0u;
+        const uint32_t row = i < n ? list[i] : 0u;
         const float4 md = a.cmeta[row];   // {error bound, scale, norm term, 0}
         const float raw = approx_raw<PREC, G>(a, q, row, t, md.y);
         const float lb = filter_lb(a.D.metric, raw, md.x, qn, md.z, a.D.d, a.D.ld);
-        const float got = __shfl_sync(FULL, lb, (int)(G * (my % PER)));
-        if (cand && my / PER == base / PER) mine = got;
+        const float got = __shfl_sync(FULL, lb, (int)(G * (lane % PER)));
+        if ((uint32_t)lane / PER == base / PER) mine = got;
     }
     return mine;
 }
@@ -331,7 +328,9 @@ __global__ void __launch_bounds__(MB == 9 ? 128 : 256, MB) search_kernel(SearchA
         const uint32_t K = a.Kq ? a.Kq[qi] : a.K;
         const uint32_t P = a.Pq ? a.Pq[qi] : a.P;
         const uint32_t T = a.T;
-        const uint32_t S = a.S;
+        const uint32_t S = min(a.S, 0x10000u);   // an expansion has at most 65535 neighbours (NeighborX::M)
+        // x / S by multiplication, exact for x < 2^16 and 2 <= S <= 2^16
+        const uint32_t inv_S = S > 1 ? 0xFFFFFFFFu / S + 1 : 0u;
         const uint32_t cap = K + P + 1;   // knn.size(), kgraph.cpp:434
 
         // query -> smem, and its norm term (SearchOracle ctor, python-api.cpp:98-101).  The padding
@@ -437,17 +436,30 @@ __global__ void __launch_bounds__(MB == 9 ? 128 : 256, MB) search_kernel(SearchA
             // once, so the walk ends; the bound only turns a defect into an error.
             const uint64_t step_limit = 64ull * (N + cap) + 4096;
             uint64_t steps = 0;
-            // The expansion loop of kgraph.cpp:478-514.  The entry at k is expanded
-            // batch after batch (S neighbours each) exactly as the reference's loop
-            // does while no insert lands at or before k.  Its adjacency entries come
-            // in windows of up to 128 (four per lane) with one round trip for the
-            // ids and one for their visited bits (this warp's private set, so the
-            // bits can only change by this walk); a batch's unvisited neighbours are
-            // then confirmed with an atomic test-and-set (exact even when an id
-            // recurs across chunks), their distances computed and inserted in one
-            // merge.  When an insert lands at or before k the reference moves on to
-            // another entry: so does this loop, and the window is dropped (it is
-            // reloaded from m when the entry comes up again).
+            // The expansion loop of kgraph.cpp:478-514.  The reference expands the entry
+            // at k batch after batch (S neighbours each) while no insert of a batch
+            // lands at or before k, else it moves on to another entry after the batch.
+            // Here an entry's adjacency comes in windows of up to 128 ids (four per
+            // lane; one round trip for the ids, one for their visited bits -- this
+            // warp's private set, so only this walk changes them), whose unvisited
+            // neighbours form a list in order.  Batches without one change nothing but
+            // the entry's progress and cost nothing.  The others are taken in groups of up
+            // to 32 candidates, whatever batches they belong to: one round trip confirms
+            // the group's candidates with an atomic test-and-set and brings their rows,
+            // and their insertion positions show the first batch with an insert at or
+            // before k.  The batches up to that one are merged into the pool in one
+            // step; the candidates after it are put back to unvisited, as the reference
+            // has not reached them (their rows were read for nothing).
+            // What bounds it: a chain of dependent round trips per entry (ids, bits,
+            // rows), so trips are what counts, not the rows' bytes.  Against one trip per
+            // batch of S (1M x 128 mixture, 10k queries, K=10): P=1000 78.2 -> 45.7 ms,
+            // 3 good starting points and P=5 5.62 -> 4.43 ms; one query on 100k x 16
+            // 1.33 -> 0.79 ms.  Groups bounded to 8 or 16 candidates were slower
+            // everywhere (49.2 / 47.1 ms, 4.98 / 4.77 ms, 1.03 / 0.88 ms).
+            if (S == 0 && L > 0 && warp_next_flagged(s.pid, 0, L, lane) < L) {   // the reference would not end
+                if (lane == 0) raise_error(a.err, ERR_STEP_LIMIT);
+                L = 0;
+            }
             while (true) {
                 k = warp_next_flagged(s.pid, k, L, lane);
                 if (k >= L) break;
@@ -474,168 +486,174 @@ __global__ void __launch_bounds__(MB == 9 ? 128 : 256, MB) search_kernel(SearchA
                     eM = mM0 >> 16;
                     m = mM0 & 0xFFFFu;
                 }
-                uint32_t wlo = 0, whi = 0;   // loaded window [wlo, whi)
-                bool wuv[4];
-                bool moved = false;
+                uint32_t wlo = m, whi = m;     // loaded window [wlo, whi)
+                uint32_t lb = 0, nl = 0;       // its unvisited neighbours not yet taken: list entries [lb, nl)
+                uint32_t lim = eM;             // end of the positions to read: after an insert at or before k,
+                bool moved = false;            //  the end of its batch
+                uint32_t endM = eM;            // the entry's progress when the walk leaves it
+                bool done = true;              // every neighbour read
                 while (true) {
-                    if (++steps > step_limit) {
-                        if (lane == 0) raise_error(a.err, ERR_STEP_LIMIT);
-                        k = L;
-                        break;
+                    if (lb >= nl) {   // the next window
+                        if (whi >= lim) break;
+                        if (++steps > step_limit) {
+                            if (lane == 0) raise_error(a.err, ERR_STEP_LIMIT);
+                            k = L;
+                            break;
+                        }
+                        wlo = whi;
+                        whi = min(wlo + 128u, lim);
+                        bool wuv[4];
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            const uint32_t p = wlo + 32 * c + lane;
+                            const bool act = p < whi;
+                            if (!act) wid[c] = 0xFFFFFFFFu;
+                            else if (!(CP && pre && p < a.ell_w)) wid[c] = neighbour(a, node, p);
+                            const bool bad = act && wid[c] >= N;
+                            if (__any_sync(FULL, bad)) { if (lane == 0) raise_error(a.err, ERR_BAD_ID); }
+                            wuv[c] = act && !bad;
+                        }
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                            if (wuv[c]) wuv[c] = !((__ldcg(vis + (wid[c] >> 5)) >> (wid[c] & 31)) & 1u);
+                        pre = false;
+                        uint32_t tot = 0;
+                        uint32_t cut = 0xFFFFFFFFu;
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            const unsigned um = __ballot_sync(FULL, wuv[c]);
+                            const uint32_t at = tot + __popc(um & ((1u << lane) - 1u));
+                            if (wuv[c]) {
+                                if (at < LIST) { s.lid[at] = wid[c]; s.lpos[at] = (uint8_t)(32 * c + lane); }
+                                else if (at == LIST) cut = wlo + 32 * c + lane;
+                            }
+                            tot += __popc(um);
+                        }
+                        if (tot > LIST) whi = __reduce_min_sync(FULL, cut);   // the rest comes with the next window
+                        lb = 0;
+                        nl = min(tot, LIST);
+                        __syncwarp();
+                        continue;
                     }
-                    // kgraph.cpp:485-491: the entry's next batch
-                    const uint32_t beginM = m;
-                    uint32_t endM = beginM + S;
-                    const bool done = endM > eM;
-                    if (done) endM = eM;
+                    // the group: lane j holds list entry lb + j, in its batch b
+                    const uint32_t c = min(nl - lb, 32u);
+                    const uint32_t at = lb + min((uint32_t)lane, c - 1);
+                    const uint32_t id = s.lid[at];
+                    const uint32_t x = wlo + s.lpos[at] - m;
+                    const uint32_t b = S == 1 ? x : __umulhi(x, inv_S);
+                    const bool act = (uint32_t)lane < c && x < lim - m;
+                    const uint32_t n = __popc(__ballot_sync(FULL, act));   // act is a prefix of the lanes
+                    if (n == 0) break;   // moved, and the rest lies behind the batch
+                    const uint32_t *list = s.lid + lb;
+                    lb += n;
+                    // an id that recurs in the group: its first position only, as the reference's
+                    // in-order loop marks it visited there (kgraph.cpp:497-498)
+                    const unsigned same = __match_any_sync(FULL, act ? id : 0xFFFFFFFFu);
+                    const bool cand = act && (__ffs(same) - 1) == lane;
+                    // L2 prefetch of the rows the next groups of this window will read, behind this
+                    // group's loads
+                    if constexpr (PF > 0) {
+                        if (lane < PF * 8 && lb + lane < nl) {
+                            const uint32_t pid2 = s.lid[lb + lane];
+                            if (PREC && L == cap - 1) prefetch_crow<PREC>(a, pid2);
+                            else prefetch_row(a.D, pid2);
+                        }
+                    }
+                    // All in flight together: the exact test-and-set of the visited bit, the
+                    // candidate's {M, degree}, and its row (distance).
+                    bool isnew = false;
+                    uint32_t aM = 0;
+                    if (cand) {
+                        const uint32_t bit = 1u << (id & 31);
+                        isnew = !(atomicOr(vis + (id >> 5), bit) & bit);
+                    }
+                    float dd = 0.f;
+                    unsigned nm, im, sm = 0;   // new candidates; those that may enter the pool; those skipped
+                    const bool full = L == cap - 1;
+                    if (PREC && full) {
+                        // Full pool: the lower bound from the compressed rows drops candidates that would
+                        // land in the spare slot; the others take the FP32 distance.
+                        const float lbd = warp_list_lb<PREC, G>(a, s.q, qn, list, n, lane);
+                        const float worst = s.pd[L - 1];
+                        const bool keep = isnew && !(lbd >= worst);
+                        nm = __ballot_sync(FULL, isnew);
+                        const unsigned km = __ballot_sync(FULL, keep);
+                        sm = nm & ~km;
+                        im = 0;
+                        if (km) {
+                            if (!CP && keep) aM = actual_M(a, a.Mp, id);
+                            const uint32_t my = __popc(km & ((1u << lane) - 1u));
+                            if (keep) s.lsel[my] = (uint8_t)lane;
+                            __syncwarp();
+                            const float got = warp_list_dist<G>(a, s.q, qn, list, s.lsel, __popc(km), lane);
+                            dd = __shfl_sync(FULL, got, (int)my);
+                            im = __ballot_sync(FULL, keep && dd < worst);
+                            __syncwarp();
+                        }
+                    } else {
+                        if (!CP && cand) aM = actual_M(a, a.Mp, id);
+                        dd = warp_list_dist<G>(a, s.q, qn, list, nullptr, n, lane);
+                        nm = __ballot_sync(FULL, isnew);
+                        // A full pool takes a candidate only below its last entry: one at or
+                        // above it lands in the spare slot (kgraph.cpp:503-506), and so does
+                        // every later candidate that is not closer than it, so leaving those
+                        // out of the merge changes no position.
+                        im = full ? __ballot_sync(FULL, isnew && dd < s.pd[L - 1]) : nm;
+                    }
+                    unsigned taken = FULL;   // the lanes of the batches the reference reads
+                    if (im) {
+                        uint32_t ai, f;
+                        const uint32_t r = warp_rank_batch(s.pd, L, cap, im, dd, ai, f, lane);
+                        const unsigned hm = __ballot_sync(FULL, r <= k);
+                        if (hm && !moved) {
+                            // the expanded entry is no longer at k after this batch: its progress
+                            // is written where it still stands
+                            const uint32_t bs = __shfl_sync(FULL, b, __ffs(hm) - 1);
+                            const uint32_t end = m + (bs + 1) * S;
+                            moved = true;
+                            done = end > eM;
+                            endM = min(end, eM);
+                            lim = endM;
+                            if (lane == 0) {
+                                if constexpr (CP) {   // progress in batches of S
+                                    s.pid[k] = done ? node : (node | FLAG_BIT | ((bq + bs + 1) << a.cp_idbits));
+                                } else {
+                                    if (done) s.pid[k] = s.pid[k] & ID_MASK;
+                                    s.pm[k] = (endM & 0xFFFFu) | (eM << 16);
+                                }
+                            }
+                            taken = __ballot_sync(FULL, b <= bs);
+                            if (isnew && b > bs) atomicAnd(vis + (id >> 5), ~(1u << (id & 31)));
+                            if (im & ~taken) {
+                                im &= taken;
+                                f = warp_rank_again(im, dd, lane);
+                            }
+                            __syncwarp();
+                        }
+                        const uint32_t mr = __reduce_min_sync(FULL, ((im >> lane) & 1u) ? r : 0xFFFFFFFFu);
+                        L = warp_apply_batch(s.pd, s.pid, CP ? nullptr : s.pm, L, cap, im, ai, f, dd, id | FLAG_BIT,
+                                             aM << 16, lane);   // new entries: flag set, m = 0, M = actual_M
+                        if (mr < k) k = mr;
+                    }
+                    n_comps += __popc(nm & taken);
+                    if (PREC && full) {
+                        n_apx += __popc(nm & taken);
+                        n_skip += __popc(sm & taken);
+                    }
+                }
+                if (k >= L) break;
+                n_adj += endM - m;
+                if (!moved) {   // every neighbour read, and the entry still at k
                     if (lane == 0) {
-                        if constexpr (CP) {   // progress in batches of S: endM = (bq + 1) S unless done
-                            s.pid[k] = done ? node : (node | FLAG_BIT | ((bq + 1) << a.cp_idbits));
+                        if constexpr (CP) {
+                            s.pid[k] = node;
                         } else {
-                            if (done) s.pid[k] = s.pid[k] & ID_MASK;
-                            s.pm[k] = (endM & 0xFFFFu) | (eM << 16);
+                            s.pid[k] = s.pid[k] & ID_MASK;
+                            s.pm[k] = (eM & 0xFFFFu) | (eM << 16);
                         }
                     }
                     __syncwarp();
-                    n_adj += endM - beginM;
-                    // kgraph.cpp:495-513.  A batch of at most 32 neighbours is one unit (lane j
-                    // holds neighbour beginM + j, gathered from the window, which is reloaded
-                    // when it does not hold the whole batch); a longer batch (S > 32) goes in
-                    // pieces that stay inside one 32-entry chunk.
-                    const bool whole = endM - beginM <= 32;   // warp-uniform
-                    for (uint32_t p0 = beginM; p0 < endM;) {
-                        if (whole ? (p0 < wlo || endM > whi) : (p0 < wlo || p0 >= whi)) {   // load the window at p0
-                            wlo = p0;
-                            whi = min(p0 + 128u, eM);
-#pragma unroll
-                            for (int c = 0; c < 4; ++c) {
-                                const uint32_t p = wlo + 32 * c + lane;
-                                const bool act = p < whi;
-                                uint32_t id = 0xFFFFFFFFu;
-                                if (act) id = (CP && pre && p < a.ell_w) ? wid[c] : neighbour(a, node, p);
-                                const bool bad = act && id >= N;
-                                if (__any_sync(FULL, bad)) { if (lane == 0) raise_error(a.err, ERR_BAD_ID); }
-                                const bool ok = act && !bad;
-                                const unsigned same = __match_any_sync(FULL, id);
-                                const unsigned okm = __ballot_sync(FULL, ok);   // every lane votes
-                                wid[c] = id;
-                                wuv[c] = ok && ((__ffs(same & okm) - 1) == lane);
-                            }
-#pragma unroll
-                            for (int c = 0; c < 4; ++c)   // first occurrences not yet visited
-                                if (wuv[c]) wuv[c] = !((__ldcg(vis + (wid[c] >> 5)) >> (wid[c] & 31)) & 1u);
-                            pre = false;
-                        }
-                        const uint32_t c = (p0 - wlo) >> 5;
-                        uint32_t id = 0, p1;
-                        bool cand;
-                        if (whole) {
-                            // the batch spans window chunks c and c + 1 at most
-                            uint32_t idA = 0, idB = 0;
-                            bool uvA = false, uvB = false;
-#pragma unroll
-                            for (int cc = 0; cc < 4; ++cc) {
-                                if ((uint32_t)cc == c) { idA = wid[cc]; uvA = wuv[cc]; }
-                                if ((uint32_t)cc == c + 1) { idB = wid[cc]; uvB = wuv[cc]; }
-                            }
-                            const uint32_t pos = p0 - wlo + lane;   // window position of this lane's neighbour
-                            const int src = (int)(pos & 31);
-                            const uint32_t ia = __shfl_sync(FULL, idA, src), ib = __shfl_sync(FULL, idB, src);
-                            const bool ua = __shfl_sync(FULL, uvA, src), ub = __shfl_sync(FULL, uvB, src);
-                            const bool second = (pos >> 5) != c;
-                            id = second ? ib : ia;
-                            const bool uv = (uint32_t)lane < endM - p0 && (second ? ub : ua);
-                            // an id in both chunks: its first position only, as the reference's
-                            // in-order loop marks it visited there (kgraph.cpp:497-498)
-                            const unsigned same = __match_any_sync(FULL, uv ? id : 0xFFFFFFFFu);
-                            cand = uv && (__ffs(same) - 1) == lane;
-                            p1 = endM;
-                        } else {
-                            const uint32_t cbase = wlo + 32 * c;
-                            p1 = min(endM, cbase + 32);
-                            const uint32_t lo = p0 - cbase, hi = p1 - cbase;
-                            bool uv = false;
-#pragma unroll
-                            for (int cc = 0; cc < 4; ++cc)
-                                if ((uint32_t)cc == c) { id = wid[cc]; uv = wuv[cc]; }
-                            cand = uv && (uint32_t)lane >= lo && (uint32_t)lane < hi;
-                        }
-                        const unsigned cm = __ballot_sync(FULL, cand);
-                        // L2 prefetch of the rows the next PF batches of this entry will
-                        // read (unvisited window ids), behind this batch's loads
-                        if constexpr (PF > 0) {
-#pragma unroll
-                            for (int cc = 0; cc < 4; ++cc) {
-                                const uint32_t pos = wlo + 32 * cc + lane;
-                                if (wuv[cc] && pos >= p1 && pos < p1 + PF * S && pos < whi) {
-                                    if (PREC && L == cap - 1) prefetch_crow<PREC>(a, wid[cc]);
-                                    else prefetch_row(a.D, wid[cc]);
-                                }
-                            }
-                        }
-                        if (PREC && cm && L == cap - 1) {
-                            // Full pool: the visited test-and-set and the compressed rows in flight
-                            // together; the lower bound drops candidates that would land in the
-                            // spare slot, the others take the FP32 path below, restricted to them.
-                            bool isnew = false;
-                            if (cand) {
-                                const uint32_t bit = 1u << (id & 31);
-                                isnew = !(atomicOr(vis + (id >> 5), bit) & bit);
-                            }
-                            const float lb = warp_cand_lb<PREC, G>(a, s.q, qn, cm, cand, id, lane);
-                            const float worst = s.pd[L - 1];
-                            const bool keep = isnew && !(lb >= worst);
-                            const unsigned nm = __ballot_sync(FULL, isnew);
-                            const unsigned km = __ballot_sync(FULL, keep);
-                            n_comps += __popc(nm);
-                            n_apx += __popc(nm);
-                            n_skip += __popc(nm & ~km);
-                            if (km) {
-                                const uint32_t aM = (!CP && keep) ? actual_M(a, a.Mp, id) : 0u;
-                                const float dd = warp_cand_dist<G>(a, s.q, qn, s.cid, km, keep, id, lane);
-                                const unsigned im = __ballot_sync(FULL, keep && dd < worst);
-                                if (im) {
-                                    uint32_t mr;
-                                    L = warp_batch_insert(s.pd, s.pid, CP ? nullptr : s.pm, L, cap, im, dd, id | FLAG_BIT, aM << 16,
-                                                          &mr, lane);
-                                    if (mr <= k) moved = true;
-                                    if (mr < k) k = mr;
-                                }
-                            }
-                        } else if (cm) {
-                            // All three in flight together: the exact test-and-set of the
-                            // visited bit, the candidate's {M, degree}, and its row (distance).
-                            bool isnew = false;
-                            uint32_t aM = 0;
-                            if (cand) {
-                                const uint32_t bit = 1u << (id & 31);
-                                isnew = !(atomicOr(vis + (id >> 5), bit) & bit);
-                                if constexpr (!CP) aM = actual_M(a, a.Mp, id);
-                            }
-                            const float dd = warp_cand_dist<G>(a, s.q, qn, s.cid, cm, cand, id, lane);
-                            const unsigned nm = __ballot_sync(FULL, isnew);
-                            n_comps += __popc(nm);
-                            // A full pool takes a candidate only below its last entry: one at or
-                            // above it lands in the spare slot (kgraph.cpp:503-506), and so does
-                            // every later candidate of the batch that is not closer than it, so
-                            // leaving those out of the merge changes no position.
-                            const unsigned im =
-                                L == cap - 1 ? __ballot_sync(FULL, isnew && dd < s.pd[L - 1]) : nm;
-                            if (im) {
-                                uint32_t mr;   // new entries: flag set, m = 0, M = actual_M
-                                L = warp_batch_insert(s.pd, s.pid, CP ? nullptr : s.pm, L, cap, im, dd, id | FLAG_BIT, aM << 16,
-                                                      &mr, lane);
-                                if (mr <= k) moved = true;   // the expanded entry is no longer at k
-                                if (mr < k) k = mr;
-                            }
-                        }
-                        p0 = p1;
-                    }
-                    m = endM;
-                    ++bq;
-                    if (done || moved) break;   // the loop head picks the reference's next k
                 }
-                if (k >= L) break;
             }
             if (L > K) L = K;   // kgraph.cpp:515
             if (!have_results) {

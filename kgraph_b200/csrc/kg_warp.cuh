@@ -70,27 +70,30 @@ __device__ __forceinline__ uint32_t warp_update_knn(PD pd, PI pid, uint32_t *pm,
 }
 
 // n successive UpdateKnnList calls (kgraph.cpp:503-512) by one warp in one
-// pass.  The candidates are the lanes set in `mask`, in lane order; each such
-// lane holds its candidate's distance di, id-with-flag idf and m|M word pmv
-// (ignored when pm is null: a pool without m|M words).
-// They are inserted in order into the sorted pool pd/pid/pm of length L whose
-// capacity is cap (slot cap-1 is the overflow slot), L growing by one per
-// candidate up to cap-1.  Their ids are distinct and absent from the pool (the
-// caller's visited set guarantees it), so the duplicate rule never fires.
-// Sequential inserts with insert-after-equals and eviction of the last entry
-// produce exactly the stable merge of the pool with the candidates ordered by
-// (distance, order), truncated to the final length; candidate i's position at
-// the moment it is inserted is a_i + #{j < i : d_j <= d_i}, a_i = #pool
-// entries <= d_i.  Returns the new L; *min_rank receives the smallest insertion
-// position among candidates that entered the list (r < L after the increment),
-// or 0xFFFFFFFF.
-__device__ __forceinline__ uint32_t warp_batch_insert(float *pd, uint32_t *pid, uint32_t *pm, uint32_t L,
-                                                      uint32_t cap, unsigned mask, float di, uint32_t idf,
-                                                      uint32_t pmv, uint32_t *min_rank, int lane) {
-    const uint32_t n = __popc(mask);
+// pass, in two steps (rank, apply).  The candidates are the lanes set in
+// `mask`, in lane order; each such lane holds its candidate's distance di,
+// id-with-flag idf and m|M word pmv (ignored when pm is null: a pool without
+// m|M words).  They are inserted in order into the sorted pool pd/pid/pm of
+// length L whose capacity is cap (slot cap-1 is the overflow slot), L growing
+// by one per candidate up to cap-1.  Their ids are distinct and absent from
+// the pool (the caller's visited set guarantees it), so the duplicate rule
+// never fires.  Sequential inserts with insert-after-equals and eviction of
+// the last entry produce exactly the stable merge of the pool with the
+// candidates ordered by (distance, order), truncated to the final length;
+// candidate i's position at the moment it is inserted is
+// a_i + #{j < i : d_j <= d_i}, a_i = #pool entries <= d_i -- which no later
+// candidate changes, so a caller may rank a run of candidates and then apply
+// any prefix of it.
+//
+// warp_rank_batch returns this lane's insertion position if its candidate
+// enters the list (r < L after the increment), else 0xFFFFFFFF; ai and f (the
+// candidates of `mask` before it in the merged order) are what the apply step
+// takes.
+__device__ __forceinline__ uint32_t warp_rank_batch(const float *pd, uint32_t L, uint32_t cap, unsigned mask, float di,
+                                                    uint32_t &ai, uint32_t &f, int lane) {
     const bool me = (mask >> lane) & 1u;
     const uint32_t my = __popc(mask & ((1u << lane) - 1u));   // this lane's candidate index
-    uint32_t ai = 0;
+    ai = 0;
     if (me) {   // upper bound of di in pd[0, L)
         uint32_t lo = 0, hi = L;
         while (lo < hi) {
@@ -99,47 +102,74 @@ __device__ __forceinline__ uint32_t warp_batch_insert(float *pd, uint32_t *pid, 
         }
         ai = lo;
     }
-    uint32_t e = 0, f = 0, mina = me ? ai : 0xFFFFFFFFu;
+    uint32_t e = 0;
+    f = 0;
     for (unsigned rest = mask; rest; rest &= rest - 1) {
         const int src = __ffs(rest) - 1;
         const float dj = __shfl_sync(FULL, di, src);
-        const uint32_t j = __popc(mask & ((1u << src) - 1u));
-        if (j < my && dj <= di) ++e;
-        if (dj < di || (dj == di && j < my)) ++f;
+        if (dj < di || (dj == di && src < lane)) ++f;
+        if (dj <= di && src < lane) ++e;
     }
     const uint32_t r = ai + e;   // position when this candidate is inserted
-    const bool ins = me && r < min(L + my + 1, cap - 1);
-    uint32_t mr = ins ? r : 0xFFFFFFFFu;
-    for (int o = 16; o; o >>= 1) {
-        mr = min(mr, __shfl_xor_sync(FULL, mr, o));
-        mina = min(mina, __shfl_xor_sync(FULL, mina, o));
+    return (me && r < min(L + my + 1, cap - 1)) ? r : 0xFFFFFFFFu;
+}
+
+// f over the candidates of `mask` alone (a prefix of the ranked run).
+__device__ __forceinline__ uint32_t warp_rank_again(unsigned mask, float di, int lane) {
+    uint32_t f = 0;
+    for (unsigned rest = mask; rest; rest &= rest - 1) {
+        const int src = __ffs(rest) - 1;
+        const float dj = __shfl_sync(FULL, di, src);
+        if (dj < di || (dj == di && src < lane)) ++f;
     }
-    *min_rank = mr;
-    const uint32_t Lf = min(L + n, cap - 1);
-    // move pool entries q >= mina up by #{j : a_j <= q}, top-down (each chunk's
-    // loads precede the next chunk's stores, which reach at most this chunk).
-    // For the chunk [top - 31, top]: the candidates with a_j <= top - 31 count
-    // for every lane (one ballot); only those with a_j inside the chunk are
-    // compared lane by lane.
-    for (int top = (int)L - 1; top >= (int)mina; top -= 32) {
-        const int q = top - lane;
-        const bool act = q >= (int)mina;
-        float dv = 0.f;
-        uint32_t iv = 0, mv = 0;
-        if (act) { dv = pd[q]; iv = pid[q]; if (pm) mv = pm[q]; }
-        const int bot = top - 31;
-        const unsigned below = __ballot_sync(FULL, me && (int)ai <= bot);
-        uint32_t sh = __popc(below);
-        for (unsigned rest = __ballot_sync(FULL, me && (int)ai > bot && (int)ai <= top); rest; rest &= rest - 1)
-            sh += (__shfl_sync(FULL, ai, __ffs(rest) - 1) <= (uint32_t)q) ? 1u : 0u;
+    return f;
+}
+
+// Merges the ranked candidates of `mask` into the pool; returns the new L.
+__device__ __forceinline__ uint32_t warp_apply_batch(float *pd, uint32_t *pid, uint32_t *pm, uint32_t L, uint32_t cap,
+                                                     unsigned mask, uint32_t ai, uint32_t f, float di, uint32_t idf,
+                                                     uint32_t pmv, int lane) {
+    const bool me = (mask >> lane) & 1u;
+    const uint32_t mina = __reduce_min_sync(FULL, me ? ai : 0xFFFFFFFFu);
+    const uint32_t Lf = min(L + (uint32_t)__popc(mask), cap - 1);
+    // move pool entries q >= mina up by #{j : a_j <= q}, top-down, 64 per step (two per lane, their
+    // loads in flight together; a step's loads precede its stores, which reach at most this step).
+    // The candidates with a_j at or below the step's bottom count for every lane (one ballot); only
+    // those with a_j inside the step are compared lane by lane.
+    for (int top = (int)L - 1; top >= (int)mina; top -= 64) {
+        const int q0 = top - lane, q1 = q0 - 32;
+        const bool act0 = q0 >= (int)mina, act1 = q1 >= (int)mina;
+        float d0 = 0.f, d1 = 0.f;
+        uint32_t i0 = 0, i1 = 0, m0 = 0, m1 = 0;
+        if (act0) { d0 = pd[q0]; i0 = pid[q0]; if (pm) m0 = pm[q0]; }
+        if (act1) { d1 = pd[q1]; i1 = pid[q1]; if (pm) m1 = pm[q1]; }
+        const int bot = top - 63;
+        uint32_t s0 = __popc(__ballot_sync(FULL, me && (int)ai <= bot)), s1 = s0;
+        for (unsigned rest = __ballot_sync(FULL, me && (int)ai > bot && (int)ai <= top); rest; rest &= rest - 1) {
+            const int aj = (int)__shfl_sync(FULL, ai, __ffs(rest) - 1);
+            s0 += aj <= q0 ? 1u : 0u;
+            s1 += aj <= q1 ? 1u : 0u;
+        }
         __syncwarp();
-        if (act && (uint32_t)q + sh < Lf) { pd[q + sh] = dv; pid[q + sh] = iv; if (pm) pm[q + sh] = mv; }
+        if (act0 && (uint32_t)q0 + s0 < Lf) { pd[q0 + s0] = d0; pid[q0 + s0] = i0; if (pm) pm[q0 + s0] = m0; }
+        if (act1 && (uint32_t)q1 + s1 < Lf) { pd[q1 + s1] = d1; pid[q1 + s1] = i1; if (pm) pm[q1 + s1] = m1; }
     }
     __syncwarp();
     const uint32_t fpos = ai + f;
     if (me && fpos < Lf) { pd[fpos] = di; pid[fpos] = idf; if (pm) pm[fpos] = pmv; }
     __syncwarp();
     return Lf;
+}
+
+// Both steps for all of `mask`; *min_rank receives the smallest insertion
+// position among candidates that entered the list, or 0xFFFFFFFF.
+__device__ __forceinline__ uint32_t warp_batch_insert(float *pd, uint32_t *pid, uint32_t *pm, uint32_t L,
+                                                      uint32_t cap, unsigned mask, float di, uint32_t idf,
+                                                      uint32_t pmv, uint32_t *min_rank, int lane) {
+    uint32_t ai, f;
+    const uint32_t r = warp_rank_batch(pd, L, cap, mask, di, ai, f, lane);
+    *min_rank = __reduce_min_sync(FULL, r);
+    return warp_apply_batch(pd, pid, pm, L, cap, mask, ai, f, di, idf, pmv, lane);
 }
 
 // First index >= k in [0, L) whose flag bit is set; L if none.
