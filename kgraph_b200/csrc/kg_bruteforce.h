@@ -9,9 +9,8 @@ namespace kgb {
 
 constexpr uint32_t BF_MAX_K = 128;   // K the tensor-core path keeps per query (larger K: the CUDA-core scan)
 
-// Whether the tensor-core path serves K on this context's dataset (shared memory fits).
+// Whether the tensor-core path serves K on this context's dataset.
 bool bruteforce_tc_supported(const kg_ctx *ctx, uint32_t K);
-size_t bruteforce_tc_smem(uint32_t ld, uint32_t K);
 // The dataset's BF16 rows and row terms (once per dataset version).
 int bruteforce_prepare(kg_ctx *ctx);
 // SearchOracle::search (kgraph.cpp:231-252) for nq device queries (rows of q_ld

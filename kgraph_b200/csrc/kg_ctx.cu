@@ -509,7 +509,7 @@ int search_locked(kg_ctx *ctx, const float *queries, size_t nq, size_t q_stride_
         bf_all = true;
         for (size_t i = 0; i < Q && bf_all; ++i) bf_all = hP[i] >= N;
     }
-    const bool use_tc_bf = bf_all && !K_per_q && ctx->bf_mode != KG_BRUTEFORCE_SCAN &&
+    bool use_tc_bf = bf_all && !K_per_q && ctx->bf_mode != KG_BRUTEFORCE_SCAN &&
                            bruteforce_tc_supported(ctx, params->K) &&
                            (ctx->bf_mode == KG_BRUTEFORCE_TENSOR || N >= 1024) && N == ctx->n;
     ctx->last_bf = kg_bruteforce_stats{};
@@ -517,6 +517,7 @@ int search_locked(kg_ctx *ctx, const float *queries, size_t nq, size_t q_stride_
     if (use_tc_bf) {   // the dataset's BF16 rows: once per dataset, outside the timed region
         const int pr = bruteforce_prepare(ctx);
         if (pr != KG_OK) return pr;
+        use_tc_bf = ctx->bf_usable;
     }
     cudaEventRecord(ctx->ev0, ctx->stream);
     if (use_tc_bf) {

@@ -97,10 +97,13 @@ struct kg_ctx {
     size_t offer_cap = 0;             // record-buffer capacity of deferred inserts, in offers (0: automatic)
     bool join_tile = true;            // FP32 join with each node's lists staged in shared memory
     kg_join_stats last_join{};
-    // tensor-core brute force (kg_bruteforce.cu): BF16 centred rows, row terms, mean + extents, work space
+    // tensor-core brute force (kg_bruteforce.cu): BF16 centred rows in the spread order (position p holds
+    // row p * bf_mult mod n), their norm columns, mean + extents, work space
     kgb::DevBuf bf_rows, bf_meta, bf_aux, bf_work;
     uint64_t bf_data_version = ~0ull;
-    float bf_ext[5] = {0, 0, 0, 0, 0};
+    float bf_ext[4] = {0, 0, 0, 0};
+    uint64_t bf_mult = 1;
+    bool bf_usable = true;           // false: the data leave no error margin (NaN, infinity)
     int bf_mode = KG_BRUTEFORCE_AUTO;
     unsigned long long *bf_stats_dev = nullptr;
     kg_bruteforce_stats last_bf{};

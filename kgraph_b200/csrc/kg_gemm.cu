@@ -566,11 +566,10 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     return fn;
 }
 
-// Tensor map of a row-major BF16 matrix (outer rows of `inner` elements, `ld`
-// apart) with a box of box_inner x box_outer and the 128-byte swizzle.  False
-// when TMA cannot address it (alignment) or the driver refuses it.
-bool bf16_map(CUtensorMap *m, const void *base, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner,
-              uint32_t box_outer) {
+}  // namespace
+
+bool tc_bf16_map(CUtensorMap *m, const void *base, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner,
+                 uint32_t box_outer, CUtensorMapSwizzle swizzle) {
     PFN_cuTensorMapEncodeTiled_v12000 fn = encode_fn();
     if (!fn || (reinterpret_cast<uintptr_t>(base) & 15) || (ld * 2) % 16 || inner == 0 || outer == 0) return false;
     const cuuint64_t dims[2] = {inner, outer};
@@ -578,16 +577,18 @@ bool bf16_map(CUtensorMap *m, const void *base, uint64_t inner, uint64_t outer, 
     const cuuint32_t box[2] = {box_inner, box_outer};
     const cuuint32_t es[2] = {1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, es,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+
+namespace {
 
 // Map of an operand as the TMA kernel reads it: K-major (op() rows x K, K
 // contiguous) -> boxes of 64 (K) x 128 rows; MN-major (stored K x MN) -> boxes
 // of 64 (MN) x 64 (K).
 bool operand_map(CUtensorMap *m, const void *X, int ld, int mn_major, int rows, int K) {
-    return mn_major ? bf16_map(m, X, (uint64_t)rows, (uint64_t)K, (uint64_t)ld, 64, 64)
-                    : bf16_map(m, X, (uint64_t)K, (uint64_t)rows, (uint64_t)ld, 64, 128);
+    return mn_major ? tc_bf16_map(m, X, (uint64_t)rows, (uint64_t)K, (uint64_t)ld, 64, 64)
+                    : tc_bf16_map(m, X, (uint64_t)K, (uint64_t)rows, (uint64_t)ld, 64, 128);
 }
 
 // Opts a kernel into more than 48 KB of dynamic shared memory, once per device,

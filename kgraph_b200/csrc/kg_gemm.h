@@ -1,6 +1,7 @@
 // Tensor-core GEMM for the router (kg_gemm.cu).
 #pragma once
 #include <cstdint>
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -17,6 +18,13 @@ void tc_gemm(cudaStream_t st, int M, int N, int K, const __nv_bfloat16 *A, int l
              size_t ws_bytes, uint32_t *err);
 // Scratch bytes tc_gemm uses for its K split of an M x N x K product (0: not split).
 size_t tc_gemm_workspace_bytes(int M, int N, int K);
+
+// Tensor map of a row-major BF16 matrix (outer rows of `inner` elements, `ld`
+// apart) with a box of box_inner x box_outer and the 128-byte swizzle (or the
+// one given).  False when TMA cannot address it (alignment) or the driver
+// refuses it.
+bool tc_bf16_map(CUtensorMap *m, const void *base, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner,
+                 uint32_t box_outer, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B);
 
 // k-means assignment on tcgen05: lab[r] = argmin_c cn[c] - 2 F[r].cent[c]
 // (ties: smaller c), best[r] that value; F is n x D, cent C x D (BF16,
