@@ -1523,10 +1523,6 @@ extern "C" int kg_build(kg_ctx *ctx, const kg_index_params *params, kg_index_inf
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e, "update");
     ctx->last_build_graph_launches = graph_launches;
 
-    ctx->joinq.release();   // the candidate queue is only needed while joining
-    ctx->joinaux.release();
-    ctx->joinb.release();
-
     // finalize (kgraph.cpp:975-988) into the context's CSR graph
     DevBuf &cnt = ctx->build_scratch[22];
     if ((e = cnt.reserve((n + 1) * 8)) != cudaSuccess) return cuda_fail(ctx, e, "alloc");

@@ -18,6 +18,12 @@
 //   3. Each epilogue thread owns one U row (one TMEM lane) and derives the
 //      approximate distance of each of its pairs: euclidean h_u + h_j - g,
 //      l2sqr twice that, angular -(g + c_u + c_j + |x_n|^2) / (n_u n_j + eps).
+//      The test is arranged so that a pair costs a dozen multiply-adds
+//      (filter_terms): with a square root and a division per pair this epilogue
+//      was two thirds of the kernel (200k x 96 unit-norm mixture, K=50 L=100
+//      S=12, whole build 386 -> 193 ms; E4M3 tiles 551 -> 345 ms), and the two
+//      warps of a lane quadrant take alternating 16-column pieces, so both work
+//      where a node has at most 32 new entries.
 //      A pair whose approximate distance minus a rigorous error margin E is
 //      above BOTH endpoints' radius cannot pass the reference's unlocked
 //      radius test (kgraph.cpp:725, radii only shrink during a join), so it is
@@ -47,7 +53,7 @@
 namespace kgb {
 namespace {
 
-constexpr int TC_THREADS = 256;          // 8 warps: warp w reads TMEM lanes 32*(w%4).., columns 64*(w/4)..
+constexpr int TC_THREADS = 256;          // 8 warps: warp w reads TMEM lanes 32*(w%4).., columns 16*(2k + w/4)..
 constexpr uint32_t TC_M = 128;           // U rows per tile = TMEM lanes
 constexpr uint32_t TC_N = 128;           // new columns per tile = TMEM columns
 constexpr uint32_t TC_TMEM_COLS = 128;
@@ -107,10 +113,35 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 struct TcShared {
     uint8_t *bbuf, *abuf;   // two 128-row tiles (BF16 or E4M3), K-major core-matrix layout
     float *xn;              // x_n, FP32
-    uint32_t *uid;          // U ids (NO_ID for a bad id)
-    float *ht, *cc, *nu, *rad;   // per U row: h, c, canonical norm term, radius snapshot
-    float *scl, *rel;       // E4M3 tiles: per U row the scale and ||v - scale q|| / ||v||
+    float4 *tA;             // per U row {A, s, radius, id (NO_ID for a bad id)} (filter_terms)
+    float2 *tC;             // {C, canonical norm term}
+    float2 *tF;             // E4M3 tiles: {scale, 1 + rel}, rel = ||v - scale q|| / ||v||
 };
+constexpr uint32_t TC_PAD = 16;   // the epilogue reads columns 16 at a time, past the last row
+
+// The filter's test, approx d - E > max radius, without a square root or a
+// division per pair: both sides times the denominator (angular), the margin's
+// terms split into one part per row, |x_u - x_n| |x_j - x_n| = s_u s_j with
+// s = sqrt(2 h) per row.
+// euclidean and l2sqr (halved): A_u + A_j - g - 2 et s_u s_j > max radius;
+// angular, full = g + A_u + A_j, w = n_u n_j:
+//   -full - 2 et s_u s_j - C_u - C_j - 2 gam w - 4 gam |full| - 4.8e-7 |g|
+//   > max radius (w + FLT_EPSILON).
+// Its rounding is a few parts in 2^24 of the same terms, inside the factor 2 of E.
+// h = |x_u - x_n|^2 / 2, c = (x_u - x_n) . x_n, qn = |x_n|^2.
+__device__ __forceinline__ void filter_terms(int metric, float h, float c, float nrm, float qn, float gam, float rad,
+                                             uint32_t id, float4 &tA, float2 &tC) {
+    const float sr = sqrtf(2.0f * h);
+    tC = make_float2(0.f, nrm);
+    if (metric == METRIC_ANGULAR) {
+        tA = make_float4(c + 0.5f * qn, sr, rad, __uint_as_float(id));
+        tC.x = 2.0f * (gam * sr * sqrtf(qn) + 0.5f * gam * qn + 2.4e-7f * (fabsf(c) + 0.5f * qn));
+    } else if (metric == METRIC_L2SQR) {   // everything halved (the radius exactly)
+        tA = make_float4(h - 6.0f * gam * h, sr, 0.5f * rad, __uint_as_float(id));
+    } else {
+        tA = make_float4(h - 2.0f * gam * h - 4.0f * gam * nrm, sr, rad, __uint_as_float(id));
+    }
+}
 
 // Rows [u0, u0 + rows) of U into `buf` (all 128 tile rows written; rows past
 // `rows` are zero).  Warp w stages row groups w, w+8: lane l owns row
@@ -118,7 +149,7 @@ struct TcShared {
 // store covers one contiguous 128-byte core matrix.
 template <int PREC>
 __device__ void stage_rows(const BuildState &s, const TcShared &sh, uint8_t *buf, uint32_t u0, uint32_t rows,
-                           int warp, int lane);
+                           float qn, float gam, int warp, int lane);
 
 // E4M3 rows with a per-row scale: v = x_u - x_n in FP32 (as the BF16 rows),
 // scale = max|v| / 448, q = e4m3_satfinite(v / scale); per row the exact
@@ -127,12 +158,12 @@ __device__ void stage_rows(const BuildState &s, const TcShared &sh, uint8_t *buf
 // (l >> 3) + 4i; the row's maximum needs a first pass over its elements.
 template <>
 __device__ void stage_rows<1>(const BuildState &s, const TcShared &sh, uint8_t *buf, uint32_t u0, uint32_t rows,
-                              int warp, int lane) {
+                              float qn, float gam, int warp, int lane) {
     const uint32_t Dp = s.D.ld, nk16 = Dp >> 4;
     for (uint32_t g = warp; g * 8 < rows; g += TC_THREADS / 32) {
         const uint32_t rl = g * 8 + (lane & 7);
         const bool valid = rl < rows;
-        const uint32_t id = valid ? sh.uid[u0 + rl] : NO_ID;
+        const uint32_t id = valid ? __float_as_uint(sh.tA[u0 + rl].w) : NO_ID;
         const bool ok = id != NO_ID;
         float nrm = 0.f, rd = -FLT_MAX;
         if (ok && lane < 8) {
@@ -184,13 +215,10 @@ __device__ void stage_rows<1>(const BuildState &s, const TcShared &sh, uint8_t *
         err2 += __shfl_xor_sync(FULL, err2, 16);
         if (lane < 8 && valid) {
             const uint32_t u = u0 + rl;
-            sh.ht[u] = 0.5f * hs;
-            sh.cc[u] = cs;
-            sh.nu[u] = nrm;
-            sh.rad[u] = rd;
-            sh.scl[u] = scale;
+            filter_terms(s.D.metric, 0.5f * hs, cs, nrm, qn, gam, rd, id, sh.tA[u], sh.tC[u]);
             // relative to ||v|| (hs carries an FP32 rounding: one more relative step of slack)
-            sh.rel[u] = hs > 0.f ? __double2float_ru(sqrt(err2) / sqrt((double)hs) * (1.0 + 1e-5)) : 0.f;
+            const float rel = hs > 0.f ? __double2float_ru(sqrt(err2) / sqrt((double)hs) * (1.0 + 1e-5)) : 0.f;
+            sh.tF[u] = make_float2(scale, 1.f + rel);
         }
     }
     tc::fence_async_shared();   // make the generic-proxy stores visible to the MMA
@@ -198,14 +226,14 @@ __device__ void stage_rows<1>(const BuildState &s, const TcShared &sh, uint8_t *
 
 template <>
 __device__ void stage_rows<0>(const BuildState &s, const TcShared &sh, uint8_t *buf, uint32_t u0, uint32_t rows,
-                              int warp, int lane) {
+                              float qn, float gam, int warp, int lane) {
     const uint32_t Dp = s.D.ld, nk8 = Dp >> 3;
     // Rows past `rows` are left as they are: the MMA reads them, but their
     // products land only in masked rows / columns of the accumulator.
     for (uint32_t g = warp; g * 8 < rows; g += TC_THREADS / 32) {
         const uint32_t rl = g * 8 + (lane & 7);
         const bool valid = rl < rows;
-        const uint32_t id = valid ? sh.uid[u0 + rl] : NO_ID;
+        const uint32_t id = valid ? __float_as_uint(sh.tA[u0 + rl].w) : NO_ID;
         const bool ok = id != NO_ID;
         float nrm = 0.f, rd = -FLT_MAX;
         if (ok && lane < 8) {   // issued ahead of the row loads
@@ -242,10 +270,7 @@ __device__ void stage_rows<0>(const BuildState &s, const TcShared &sh, uint8_t *
         cs += __shfl_xor_sync(FULL, cs, 16);
         if (lane < 8 && valid) {
             const uint32_t u = u0 + rl;
-            sh.ht[u] = 0.5f * hs;
-            sh.cc[u] = cs;
-            sh.nu[u] = nrm;
-            sh.rad[u] = rd;
+            filter_terms(s.D.metric, 0.5f * hs, cs, nrm, qn, gam, rd, id, sh.tA[u], sh.tC[u]);
         }
     }
     tc::fence_async_shared();   // make the generic-proxy stores visible to the MMA
@@ -260,7 +285,6 @@ __global__ void __launch_bounds__(TC_THREADS, 3) join_tc_kernel(BuildState s, ui
     __shared__ uint32_t s_list[TC_CLAIM], s_la[TC_CLAIM], s_lb[TC_CLAIM];
     __shared__ uint32_t s_wcnt[TC_THREADS / 32];
     __shared__ unsigned long long s_wbase[TC_THREADS / 32];
-    __shared__ float s_qn;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t Dp = s.D.ld, N = s.D.n;
     const uint32_t n_begin = jq.bounds[round], n_end = jq.bounds[round + 1];
@@ -269,13 +293,9 @@ __global__ void __launch_bounds__(TC_THREADS, 3) join_tc_kernel(BuildState s, ui
     sh.bbuf = smem;
     sh.abuf = smem + tile_bytes;
     sh.xn = reinterpret_cast<float *>(smem + 2 * tile_bytes);
-    sh.uid = reinterpret_cast<uint32_t *>(sh.xn + Dp);
-    sh.ht = reinterpret_cast<float *>(sh.uid + Umax);
-    sh.cc = sh.ht + Umax;
-    sh.nu = sh.cc + Umax;
-    sh.rad = sh.nu + Umax;
-    sh.scl = sh.rad + Umax;
-    sh.rel = sh.scl + Umax;
+    sh.tA = reinterpret_cast<float4 *>(sh.xn + Dp);   // 16-byte aligned: Dp is a multiple of 16
+    sh.tC = reinterpret_cast<float2 *>(sh.tA + Umax + TC_PAD);
+    sh.tF = sh.tC + Umax + TC_PAD;
 
     if (warp == 0) tc::tmem_alloc(&tmem_base, TC_TMEM_COLS);
     if (tid == 0) tc::mbar_init(&mbar, 1);
@@ -291,9 +311,7 @@ __global__ void __launch_bounds__(TC_THREADS, 3) join_tc_kernel(BuildState s, ui
     const int metric = s.D.metric;
     uint32_t phase = 0;
     bool aborted = false;
-    unsigned long long comps = 0, passed = 0, sampled = 0, viol = 0, relc = 0;
-    double sum_abs = 0, sum_ratio = 0, sum_rel = 0;
-    float max_abs = 0.f, max_ratio = 0.f, max_rel = 0.f;
+    unsigned long long comps = 0, passed = 0;
 
     for (;;) {
         // claim TC_CLAIM nodes of this round's range; keep those with new entries
@@ -335,26 +353,23 @@ __global__ void __launch_bounds__(TC_THREADS, 3) join_tc_kernel(BuildState s, ui
         for (uint32_t u = tid; u < U; u += TC_THREADS) {
             uint32_t id = u < a ? nw[u] : od[u - a];
             if (id >= N) { raise_error(s.err, ERR_BAD_ID); id = NO_ID; }
-            sh.uid[u] = id;
+            sh.tA[u].w = __uint_as_float(id);
         }
         const float *xrow = s.D.X + (size_t)n * Dp;
         for (uint32_t k = tid; k < Dp; k += TC_THREADS) sh.xn[k] = xrow[k];
         __syncthreads();
-        if (warp == 0) {
-            float qs = 0.f;
-            for (uint32_t k = lane; k < Dp; k += 32) qs += sh.xn[k] * sh.xn[k];
-            for (int o = 16; o; o >>= 1) qs += __shfl_xor_sync(FULL, qs, o);
-            if (lane == 0) s_qn = qs;
-        }
+        float qn = 0.f;   // |x_n|^2, in every warp
+        for (uint32_t k = lane; k < Dp; k += 32) qn += sh.xn[k] * sh.xn[k];
+        for (int o = 16; o; o >>= 1) qn += __shfl_xor_sync(FULL, qn, o);
         const bool samp = sampled_node(n);
         for (uint32_t j0 = 0; j0 < a && !aborted; j0 += TC_N) {
             const uint32_t j1 = min(a, j0 + TC_N);
-            stage_rows<PREC>(s, sh, sh.bbuf, j0, min(U, j0 + TC_M) - j0, warp, lane);
+            stage_rows<PREC>(s, sh, sh.bbuf, j0, min(U, j0 + TC_M) - j0, qn, gam, warp, lane);
             for (uint32_t u0 = 0; u0 < U; u0 += TC_M) {
                 const uint32_t u1 = min(U, u0 + TC_M);
                 if (!(u1 > max(u0, a) || (u0 < a && u0 + 1 < j1))) continue;   // no pair needed in this tile
                 const bool same = u0 == j0;
-                if (!same) stage_rows<PREC>(s, sh, sh.abuf, u0, u1 - u0, warp, lane);
+                if (!same) stage_rows<PREC>(s, sh, sh.abuf, u0, u1 - u0, qn, gam, warp, lane);
                 tc::fence_before_sync();
                 __syncthreads();
                 if (tid == 0) {
@@ -382,100 +397,114 @@ __global__ void __launch_bounds__(TC_THREADS, 3) join_tc_kernel(BuildState s, ui
                 phase ^= 1;
                 tc::fence_after_sync();
 
-                // ---- epilogue: this thread's U row against 64 columns
+                // ---- epilogue: this thread's U row against the columns 16 (2 k + half) .. + 15
                 const uint32_t u = u0 + 32 * q + lane;
-                const bool uval = u < u1 && sh.uid[u] != NO_ID;
-                const uint32_t idu = uval ? sh.uid[u] : 0u;
+                const float4 ua = u < u1 ? sh.tA[u] : make_float4(0.f, 0.f, 0.f, __uint_as_float(NO_ID));
+                const bool uval = __float_as_uint(ua.w) != NO_ID;
+                const uint32_t idu = uval ? __float_as_uint(ua.w) : 0u;
                 const bool unew = u < a;
-                const float hu = uval ? sh.ht[u] : 0.f, cu = uval ? sh.cc[u] : 0.f, nuu = uval ? sh.nu[u] : 0.f;
-                const float radu = uval ? sh.rad[u] : -FLT_MAX;
-                const float su = (PREC == 1 && uval) ? sh.scl[u] : 1.f, ru = (PREC == 1 && uval) ? sh.rel[u] : 0.f;
-                const float qn = s_qn;
-                unsigned pmask[2] = {0u, 0u};
-                for (int part = 0; part < 2; ++part) {
-                    const uint32_t cb = 64 * half + 32 * part;
+                const float2 uc = uval ? sh.tC[u] : make_float2(0.f, 0.f);
+                const float2 uf = (PREC == 1 && uval) ? sh.tF[u] : make_float2(1.f, 1.f);
+                const float k2 = 2.f * et * ua.y;
+                const bool wnew = u0 + 32 * q < a;   // the warp holds new rows
+                unsigned pmask[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+                for (int part = 0; part < 4; ++part) {
+                    const uint32_t cb = 32 * part + 16 * half;
                     if (j0 + cb >= j1) break;   // warp-uniform
-                    float v[32];
-                    tc::tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + cb, v);
+                    float v[16];
+                    tc::tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + cb, v);
+                    // the pairs of this row: columns in range, after the row among the new ones
+                    const uint32_t cols = min(16u, j1 - j0 - cb);
+                    unsigned need = uval ? (1u << cols) - 1u : 0u;
+                    if (unew && u >= j0 + cb) need &= u - j0 - cb >= 15 ? 0u : ~0u << (u - j0 - cb + 1);
                     unsigned pm = 0;
 #pragma unroll
-                    for (int c = 0; c < 32; ++c) {
-                        const uint32_t j = j0 + cb + c;
-                        const uint32_t idj = j < j1 ? sh.uid[j] : NO_ID;
-                        const bool need = uval && idj != NO_ID && (!unew || (j > u && idj != idu));
-                        if (need) {
-                            ++comps;
-                            float gv = v[c], etp = et;
-                            if constexpr (PREC == 1) {   // the scales, and this pair's relative error
-                                gv = gv * su * sh.scl[j];
-                                const float rj = sh.rel[j];
-                                etp = ru + rj + ru * rj + g8 * (1.f + ru) * (1.f + rj);
-                            }
-                            const Approx ap = approx_dist(metric, gv, hu, sh.ht[j], cu, sh.cc[j], nuu, sh.nu[j],
-                                                          qn, etp, gam);
-                            if (!(ap.d - ap.e > fmaxf(radu, sh.rad[j]))) pm |= 1u << c;
+                    for (int c = 0; c < 16; ++c) {
+                        const float4 ja = sh.tA[j0 + cb + c];   // rows up to Umax: past j1 masked below
+                        float g = v[c], t2 = k2 * ja.y;
+                        if constexpr (PREC == 1) {   // the scales, and this pair's relative error
+                            const float2 jf = sh.tF[j0 + cb + c];
+                            g = g * uf.x * jf.x;
+                            t2 = 2.f * (uf.y * jf.y * (1.f + g8) - 1.f) * ua.y * ja.y;
                         }
+                        bool skip;
+                        if (metric == METRIC_ANGULAR) {
+                            const float2 jc = sh.tC[j0 + cb + c];
+                            const float full = g + (ua.x + ja.x), w = uc.y * jc.y;
+                            const float lhs = -full - t2 - (uc.x + jc.x) - 2.f * gam * w - 4.f * gam * fabsf(full) -
+                                              4.8e-7f * fabsf(g);
+                            skip = lhs > fmaxf(ua.z, ja.z) * (w + FLT_EPSILON);
+                        } else {
+                            skip = (ua.x + ja.x) - g - t2 > fmaxf(ua.z, ja.z);
+                        }
+                        if (!skip) pm |= 1u << c;
+                        const uint32_t idj = __float_as_uint(ja.w);
+                        if (idj == NO_ID || (wnew && unew && idj == idu)) need &= ~(1u << c);
                     }
+                    pm &= need;
+                    comps += __popc(need);
+                    pmask[part] = pm;
                     if (samp) {   // FP64 tile error on this node's pairs, one pair at a time per warp
-                        unsigned nm = 0;
-                        for (int c = 0; c < 32; ++c) {
-                            const uint32_t j = j0 + cb + c;
-                            const uint32_t idj = j < j1 ? sh.uid[j] : NO_ID;
-                            if (uval && idj != NO_ID && (!unew || (j > u && idj != idu))) nm |= 1u << c;
-                        }
+                        unsigned nm = need;
                         for (;;) {
                             const unsigned any = __ballot_sync(FULL, nm != 0);
                             if (!any) break;
                             const int src = __ffs(any) - 1;
                             uint32_t ia = 0, ib = 0;
-                            float apd = 0.f, ape = 0.f;
+                            float g = 0.f, etp = et;
                             if (lane == src) {
                                 const int c = __ffs(nm) - 1;
                                 nm &= nm - 1;
                                 const uint32_t j = j0 + cb + c;
-                                float g = 0.f;
 #pragma unroll
-                                for (int k = 0; k < 32; ++k) if (k == c) g = v[k];
-                                float etp = et;
+                                for (int k = 0; k < 16; ++k) if (k == c) g = v[k];
                                 if constexpr (PREC == 1) {
-                                    g = g * su * sh.scl[j];
-                                    const float rj = sh.rel[j];
-                                    etp = ru + rj + ru * rj + g8 * (1.f + ru) * (1.f + rj);
+                                    g = g * uf.x * sh.tF[j].x;
+                                    etp = uf.y * sh.tF[j].y * (1.f + g8) - 1.f;
                                 }
-                                const Approx ap = approx_dist(metric, g, hu, sh.ht[j], cu, sh.cc[j], nuu, sh.nu[j],
-                                                              qn, etp, gam);
-                                apd = ap.d;
-                                ape = ap.e;
                                 ia = idu;
-                                ib = sh.uid[j];
+                                ib = __float_as_uint(sh.tA[j].w);
                             }
                             ia = __shfl_sync(FULL, ia, src);
                             ib = __shfl_sync(FULL, ib, src);
-                            apd = __shfl_sync(FULL, apd, src);
-                            ape = __shfl_sync(FULL, ape, src);
+                            g = __shfl_sync(FULL, g, src);
+                            etp = __shfl_sync(FULL, etp, src);
+                            // h and c of both rows again (the filter keeps only what its test takes)
+                            float hc[4] = {0.f, 0.f, 0.f, 0.f};
+                            for (uint32_t k = lane; k < Dp; k += 32) {
+                                const float x = sh.xn[k], ea = s.D.X[(size_t)ia * Dp + k] - x, eb = s.D.X[(size_t)ib * Dp + k] - x;
+                                hc[0] += ea * ea; hc[1] += eb * eb; hc[2] += ea * x; hc[3] += eb * x;
+                            }
+#pragma unroll
+                            for (int k = 0; k < 4; ++k)
+                                for (int o = 16; o; o >>= 1) hc[k] += __shfl_xor_sync(FULL, hc[k], o);
+                            const Approx ap = approx_dist(metric, g, 0.5f * hc[0], 0.5f * hc[1], hc[2], hc[3],
+                                                          s.D.norms[ia], s.D.norms[ib], qn, etp, gam);
+                            const float apd = ap.d, ape = ap.e;
                             const double d64 = warp_dist64(s.D, ia, ib, lane);
                             if (lane == 0) {
                                 const double err = fabs((double)apd - d64);
                                 const double ratio = err / (double)ape;
-                                ++sampled;
-                                sum_abs += err;
-                                sum_ratio += ratio;
-                                max_abs = fmaxf(max_abs, (float)err);
-                                max_ratio = fmaxf(max_ratio, (float)ratio);
+                                // few nodes: straight to the counters, no registers held for them
+                                atomicAdd(&s.tc->sampled, 1ull);
+                                atomicAdd(&s.tc->sum_abs, err);
+                                atomicAdd(&s.tc->sum_ratio, ratio);
+                                atomicMax(&s.tc->max_abs_bits, __float_as_uint((float)err));
+                                atomicMax(&s.tc->max_ratio_bits, __float_as_uint((float)ratio));
                                 if (d64 != 0.0) {
                                     const double rel = err / fabs(d64);
-                                    ++relc;
-                                    sum_rel += rel;
-                                    max_rel = fmaxf(max_rel, (float)rel);
+                                    atomicAdd(&s.tc->rel_count, 1ull);
+                                    atomicAdd(&s.tc->sum_rel, rel);
+                                    atomicMax(&s.tc->max_rel_bits, __float_as_uint((float)rel));
                                 }
-                                if (err > (double)ape) ++viol;
+                                if (err > (double)ape) atomicAdd(&s.tc->violations, 1ull);
                             }
                         }
                     }
-                    pmask[part] = pm;
                 }
                 // append the survivors: one queue atomic per tile
-                const uint32_t mine = __popc(pmask[0]) + __popc(pmask[1]);
+                const uint32_t mine = __popc(pmask[0]) + __popc(pmask[1]) + __popc(pmask[2]) + __popc(pmask[3]);
                 uint32_t incl = mine;
                 for (int o = 1; o < 32; o <<= 1) {
                     const uint32_t t = __shfl_up_sync(FULL, incl, o);
@@ -492,13 +521,14 @@ __global__ void __launch_bounds__(TC_THREADS, 3) join_tc_kernel(BuildState s, ui
                 __syncthreads();
                 unsigned long long pos = s_wbase[warp] + incl - mine;
                 passed += mine;
-                for (int part = 0; part < 2; ++part) {
+#pragma unroll
+                for (int part = 0; part < 4; ++part) {
                     unsigned pm = pmask[part];
-                    const uint32_t cb = 64 * half + 32 * part;
+                    const uint32_t cb = 32 * part + 16 * half;
                     while (pm) {
                         const int c = __ffs(pm) - 1;
                         pm &= pm - 1;
-                        const uint32_t idj = sh.uid[j0 + cb + c];
+                        const uint32_t idj = __float_as_uint(sh.tA[j0 + cb + c].w);
                         jq.x[pos] = unew ? min(idu, idj) : idj;
                         jq.y[pos] = unew ? max(idu, idj) : idu;
                         jq.n[pos] = n;
@@ -523,30 +553,10 @@ __global__ void __launch_bounds__(TC_THREADS, 3) join_tc_kernel(BuildState s, ui
     for (int o = 16; o; o >>= 1) {
         comps += __shfl_xor_sync(FULL, comps, o);
         passed += __shfl_xor_sync(FULL, passed, o);
-        sampled += __shfl_xor_sync(FULL, sampled, o);
-        viol += __shfl_xor_sync(FULL, viol, o);
-        relc += __shfl_xor_sync(FULL, relc, o);
-        sum_abs += __shfl_xor_sync(FULL, sum_abs, o);
-        sum_ratio += __shfl_xor_sync(FULL, sum_ratio, o);
-        sum_rel += __shfl_xor_sync(FULL, sum_rel, o);
-        max_abs = fmaxf(max_abs, __shfl_xor_sync(FULL, max_abs, o));
-        max_ratio = fmaxf(max_ratio, __shfl_xor_sync(FULL, max_ratio, o));
-        max_rel = fmaxf(max_rel, __shfl_xor_sync(FULL, max_rel, o));
     }
     if (lane == 0) {
         if (comps) { atomicAdd(s.n_comps, comps); atomicAdd(&s.tc->pairs, comps); }
         if (passed) atomicAdd(&s.tc->rechecked, passed);
-        if (viol) atomicAdd(&s.tc->violations, viol);
-        if (sampled) {
-            atomicAdd(&s.tc->sampled, sampled);
-            atomicAdd(&s.tc->rel_count, relc);
-            atomicAdd(&s.tc->sum_abs, sum_abs);
-            atomicAdd(&s.tc->sum_ratio, sum_ratio);
-            atomicAdd(&s.tc->sum_rel, sum_rel);
-            atomicMax(&s.tc->max_abs_bits, __float_as_uint(max_abs));
-            atomicMax(&s.tc->max_ratio_bits, __float_as_uint(max_ratio));
-            atomicMax(&s.tc->max_rel_bits, __float_as_uint(max_rel));
-        }
     }
 }
 
@@ -614,13 +624,13 @@ __global__ void join_bounds_kernel(const uint64_t *pre, uint32_t N, uint64_t sla
 
 size_t join_tc_smem(const BuildState &s, int prec) {
     const size_t Umax = (size_t)s.NEWCAP + s.OLDCAP;
-    return 2 * (size_t)TC_M * s.D.ld * (prec ? 1 : 2) + (size_t)s.D.ld * 4 + Umax * 4 * 7;
+    return 2 * (size_t)TC_M * s.D.ld * (prec ? 1 : 2) + (size_t)s.D.ld * 4 + (Umax + TC_PAD) * (prec ? 32 : 24);
 }
 
 }  // namespace
 
 bool join_tc_supported(const BuildState &s, int prec) {
-    return s.D.ld % (prec ? 32 : 16) == 0 && join_tc_smem(s, prec) <= 200 * 1024;
+    return s.D.ld % (prec ? 32 : 16) == 0 && join_tc_smem(s, prec) <= 224 * 1024;   // with the static part, within a CTA's 227 KB
 }
 
 uint64_t join_tc_node_max(const BuildState &s) {
