@@ -6,11 +6,11 @@
 // then std::sort's each list by distance and drops ADJACENT duplicate ids.
 // std::sort is not stable, so the final order of equal distances -- and which
 // duplicates end up adjacent -- depends on the list's push order and on the
-// GNU introsort.  Here the push order is rebuilt exactly (reverse edges
-// grouped by target with a stable radix sort of (target) over edges numbered
-// in (i, j) order, the node's own forward edges spliced in at i == x), and
-// each list is sorted by the same introsort (kg_sort.h), one thread per node.
-// The result is the reference's graph bit for bit.
+// GNU introsort.  Here the push order is rebuilt exactly (reverse edges,
+// source and distance, grouped by target with a stable radix sort of (target)
+// over edges numbered in (i, j) order, the node's own forward edges spliced in
+// at i == x), and each list is sorted by the same introsort (kg_sort.h), one
+// warp per node.  The result is the reference's graph bit for bit.
 #include <cub/cub.cuh>
 #include <iostream>
 #include <vector>
@@ -31,104 +31,120 @@ __global__ void rev_count_kernel(uint32_t N, const uint64_t *off, const uint32_t
     }
 }
 
-// One entry per kept forward edge, numbered in (i, j) order: its target and index.
-__global__ void rev_edges_kernel(uint32_t N, const uint64_t *off, const uint32_t *nbr, const uint64_t *koff,
-                                 uint32_t *key, uint32_t *val, uint64_t *rc, uint32_t *err) {
+// One entry per kept forward edge, in (i, j) order: its target, and its source and distance.
+__global__ void rev_edges_kernel(uint32_t N, const uint64_t *off, const uint32_t *nbr, const float *nbr_d,
+                                 const uint64_t *koff, uint32_t *key, unsigned long long *val, uint32_t *err) {
     const int lane = threadIdx.x & 31;
     const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t i = w; i < N; i += nw) {
-        const uint64_t b = koff[i];
+        const uint64_t b = koff[i], o = off[i];
         const uint32_t k = (uint32_t)(koff[i + 1] - b);
         for (uint32_t j = lane; j < k; j += 32) {
-            uint32_t t = nbr[off[i] + j];
+            uint32_t t = nbr[o + j];
             if (t >= N) { atomicOr(err, 4u); t = i; }
             key[b + j] = t;
-            val[b + j] = (uint32_t)(b + j);
-            atomicAdd(reinterpret_cast<unsigned long long *>(rc + t), 1ull);
+            val[b + j] = (unsigned long long)__float_as_uint(nbr_d[o + j]) << 32 | i;
         }
     }
 }
 
-__global__ void rev_degree_kernel(uint32_t N, const uint64_t *kcnt, const uint64_t *rc, uint64_t *deg) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) deg[i] = kcnt[i] + rc[i];
-}
-
-// Upper bound of edge index e in the (i, j) numbering -> source node i.
-__device__ __forceinline__ uint32_t source_of(const uint64_t *koff, uint32_t N, uint64_t e) {
-    uint32_t lo = 0, hi = N;   // first i with koff[i+1] > e
-    while (lo < hi) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (koff[mid + 1] > e) hi = mid; else lo = mid + 1;
+// toff[t]: the first sorted edge whose target is t or above; toff[N] = E.
+__global__ void rev_offsets_kernel(uint32_t N, uint64_t E, const uint32_t *skey, uint64_t *toff) {
+    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e <= E; e += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t hi = e < E ? skey[e] : N;
+        for (uint32_t t = e ? skey[e - 1] + 1 : 0u; t <= hi; ++t) toff[t] = e;
     }
-    return lo;
 }
-
-struct ListAcc {
-    float *d; uint32_t *i;
-    struct Rec { float d; uint32_t i; };
-    __device__ float key(int x) const { return d[x]; }
-    __device__ void swap(int x, int y) const {
-        float td = d[x]; d[x] = d[y]; d[y] = td;
-        uint32_t ti = i[x]; i[x] = i[y]; i[y] = ti;
-    }
-    __device__ Rec get(int x) const { return Rec{d[x], i[x]}; }
-    __device__ void put(int x, Rec r) const { d[x] = r.d; i[x] = r.i; }
-    __device__ float rkey(Rec r) const { return r.d; }
-};
 
 // Rebuilds node x's list in the reference's push order, sorts it with the
-// GNU introsort, removes adjacent duplicate ids; writes its final length.
-__global__ void rev_assemble_kernel(uint32_t N, const uint64_t *off, const uint32_t *nbr, const float *nbr_d,
-                                    const uint64_t *koff, const uint64_t *toff, const uint32_t *sorted_val,
-                                    const uint64_t *noff, uint32_t *out_i, float *out_d, uint64_t *fdeg) {
-    for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < N; x += gridDim.x * blockDim.x) {
-        uint32_t *oi = out_i + noff[x];
-        float *od = out_d + noff[x];
-        uint32_t p = 0;
-        uint64_t q = toff[x];
-        const uint64_t qe = toff[x + 1];
-        const uint32_t kx = (uint32_t)(koff[x + 1] - koff[x]);
-        // reverse edges from sources i < x
-        while (q < qe) {
-            uint64_t e = sorted_val[q];
-            uint32_t src = source_of(koff, N, e);
-            if (src >= x) break;
-            oi[p] = src;
-            od[p] = nbr_d[off[src] + (e - koff[src])];
-            ++p; ++q;
+// GNU introsort, removes adjacent duplicate ids; writes its final length.  The
+// list has room at koff[x] + toff[x] of the output (every forward edge and every
+// reverse edge before it); it is sorted in shared memory up to REV_CAP entries,
+// in place beyond.  Bound: the sort's dependent steps, one warp per list.  1M
+// nodes x 40 edges, the whole call: 29.4 ms with one thread per list sorting in
+// global memory and searching each reverse edge's source; 10.1 ms now (both
+// with the import and export of the graph).
+constexpr uint32_t REV_CAP = 480;
+constexpr int REV_WARPS = 8;
+__global__ void __launch_bounds__(REV_WARPS * 32) rev_assemble_kernel(uint32_t N, const uint64_t *off, const uint32_t *nbr,
+                                                                      const float *nbr_d, const uint64_t *koff,
+                                                                      const uint64_t *toff,
+                                                                      const unsigned long long *sval, uint32_t *out_i,
+                                                                      float *out_d, uint64_t *fdeg) {
+    __shared__ float s_d[REV_WARPS][REV_CAP];
+    __shared__ uint32_t s_i[REV_WARPS][REV_CAP], s_tmp[REV_WARPS][WARP_SORT_TMP];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const unsigned ALL = 0xFFFFFFFFu, below = (1u << lane) - 1u;
+    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t x = w; x < N; x += nw) {
+        const uint64_t k0 = koff[x], q0 = toff[x], o0 = off[x];
+        const uint32_t kx = (uint32_t)(koff[x + 1] - k0), rx = (uint32_t)(toff[x + 1] - q0), p = kx + rx;
+        uint32_t *gi = out_i + k0 + q0;
+        float *gd = out_d + k0 + q0;
+        const bool in_smem = p <= REV_CAP;
+        uint32_t *li = in_smem ? s_i[wib] : gi;
+        float *ld = in_smem ? s_d[wib] : gd;
+        // reverse edges from sources below x, then (behind the node's own) from sources above it
+        uint32_t nb = 0;
+        for (uint32_t b = 0; b < rx; b += 32) {
+            const uint32_t j = b + lane;
+            const unsigned long long v = j < rx ? sval[q0 + j] : 0ull;
+            const uint32_t src = (uint32_t)v;
+            if (j < rx && src != x) {
+                const uint32_t at = src < x ? j : j + kx;
+                li[at] = src;
+                ld[at] = __uint_as_float((uint32_t)(v >> 32));
+            }
+            nb += __popc(__ballot_sync(ALL, j < rx && src < x));
         }
         // own forward edges; a self loop's reverse edge follows its forward edge
-        for (uint32_t j = 0; j < kx; ++j) {
-            oi[p] = nbr[off[x] + j];
-            od[p] = nbr_d[off[x] + j];
-            ++p;
-            while (q < qe) {
-                uint64_t e = sorted_val[q];
-                if (source_of(koff, N, e) != x || e - koff[x] != j) break;
-                oi[p] = x;
-                od[p] = nbr_d[off[x] + j];
-                ++p; ++q;
+        uint32_t ns = 0;
+        for (uint32_t b = 0; b < kx; b += 32) {
+            const uint32_t j = b + lane;
+            const uint32_t id = j < kx ? nbr[o0 + j] : 0u;
+            const unsigned self = __ballot_sync(ALL, j < kx && (id == x || id >= N));   // an id out of range was keyed to x
+            if (j < kx) {
+                const uint32_t at = nb + j + ns + __popc(self & below);
+                const float dd = nbr_d[o0 + j];
+                li[at] = id;
+                ld[at] = dd;
+                if ((self >> lane) & 1u) { li[at + 1] = x; ld[at + 1] = dd; }
             }
+            ns += __popc(self);
         }
-        // reverse edges from sources i > x
-        while (q < qe) {
-            uint64_t e = sorted_val[q];
-            uint32_t src = source_of(koff, N, e);
-            oi[p] = src;
-            od[p] = nbr_d[off[src] + (e - koff[src])];
-            ++p; ++q;
+        __syncwarp();
+        if (p <= (uint32_t)WARP_SORT_MAX) {
+            warp_gnu_sort(ld, li, nullptr, (int)p, s_tmp[wib], lane);   // kgraph.cpp:697
+        } else {
+            if (lane == 0) { WarpSortAcc acc{ld, li, nullptr}; gnu_sort(acc, 0, (int)p); }
+            __syncwarp();
         }
-        ListAcc acc{od, oi};
-        gnu_sort(acc, 0, (int)p);   // kgraph.cpp:697
-        uint32_t m = 0;             // std::unique by id (kgraph.cpp:698)
-        for (uint32_t r = 0; r < p; ++r) {
-            if (m > 0 && oi[m - 1] == oi[r]) continue;
-            oi[m] = oi[r];
-            od[m] = od[r];
-            ++m;
+        uint32_t m = 0;   // std::unique by id (kgraph.cpp:698): entries equal to the one before go
+        uint32_t last = 0;
+        for (uint32_t b = 0; b < p; b += 32) {
+            const uint32_t r = b + lane;
+            const uint32_t id = r < p ? li[r] : 0u;
+            const float dd = r < p ? ld[r] : 0.f;
+            uint32_t prev = __shfl_up_sync(ALL, id, 1);
+            if (lane == 0) prev = last;
+            last = __shfl_sync(ALL, id, 31);
+            const bool keep = r < p && (r == 0 || id != prev);
+            const unsigned km = __ballot_sync(ALL, keep);
+            if (keep) {   // at or before r, and every lane has read its entry
+                const uint32_t at = m + __popc(km & below);
+                gi[at] = id;
+                gd[at] = dd;
+            }
+            m += __popc(km);
         }
-        fdeg[x] = m;
+        if (lane == 0) fdeg[x] = m;
+        __syncwarp();
     }
+}
+
+// Like koff, the lists' places in the assembled graph: room for every edge.
+__global__ void rev_places_kernel(uint32_t N, const uint64_t *koff, const uint64_t *toff, uint64_t *noff) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= N; i += gridDim.x * blockDim.x) noff[i] = koff[i] + toff[i];
 }
 
 __global__ void compact_kernel(uint32_t N, const uint64_t *src_off, const uint64_t *dst_off, const uint32_t *si,
@@ -176,20 +192,16 @@ int graph_reverse(kg_ctx *ctx, int rev_k) {
     // re-allocating ~2 GB (1M nodes) each time costs device-synchronising cudaFree / cudaMalloc calls whose
     // time varied from build to build.  Buffers grow with 1/8 slack.
     DevBuf *R = ctx->rev_scratch;
-    DevBuf &kcnt = R[0], &koff = R[1], &rc = R[2], &toff = R[3], &deg = R[4], &noff = R[5], &fdeg = R[6],
-           &foff = R[7], &key = R[8], &val = R[9], &skey = R[10], &sval = R[11], &tmp = R[12], &ai = R[13],
-           &ad = R[14], &fi = R[15], &fd = R[16];
+    DevBuf &kcnt = R[0], &koff = R[1], &toff = R[2], &noff = R[3], &fdeg = R[4], &foff = R[5], &key = R[6], &val = R[7],
+           &skey = R[8], &sval = R[9], &tmp = R[10], &ai = R[11], &ad = R[12], &fi = R[13], &fd = R[14];
     auto grow = [](DevBuf &b, size_t bytes) { return b.reserve(bytes <= b.bytes ? bytes : bytes + bytes / 8); };
     auto fail = [&](const char *w) { return cuda_fail(ctx, e, w); };
     if ((e = grow(kcnt, (n + 1) * 8)) != cudaSuccess || (e = grow(koff, (n + 1) * 8)) != cudaSuccess ||
-        (e = grow(rc, (n + 1) * 8)) != cudaSuccess || (e = grow(toff, (n + 1) * 8)) != cudaSuccess ||
-        (e = grow(deg, (n + 1) * 8)) != cudaSuccess || (e = grow(noff, (n + 1) * 8)) != cudaSuccess ||
+        (e = grow(toff, (n + 1) * 8)) != cudaSuccess || (e = grow(noff, (n + 1) * 8)) != cudaSuccess ||
         (e = grow(fdeg, (n + 1) * 8)) != cudaSuccess || (e = grow(foff, (n + 1) * 8)) != cudaSuccess)
         return fail("alloc reverse");
-    cudaMemsetAsync(kcnt.p, 0, (n + 1) * 8, st);
-    cudaMemsetAsync(rc.p, 0, (n + 1) * 8, st);
-    cudaMemsetAsync(deg.p, 0, (n + 1) * 8, st);
-    cudaMemsetAsync(fdeg.p, 0, (n + 1) * 8, st);
+    cudaMemsetAsync(kcnt.as<uint64_t>() + n, 0, 8, st);   // the scans take one extra zero
+    cudaMemsetAsync(fdeg.as<uint64_t>() + n, 0, 8, st);
     const int grid = ctx->num_sms * 4;
     rev_count_kernel<<<grid, 256, 0, st>>>(N, ctx->offsets.as<uint64_t>(), ctx->Mnode.as<uint32_t>(), rev_k,
                                            kcnt.as<uint64_t>());
@@ -198,33 +210,32 @@ int graph_reverse(kg_ctx *ctx, int rev_k) {
     cudaMemcpyAsync(&Ef, koff.as<uint64_t>() + N, 8, cudaMemcpyDeviceToHost, st);
     cudaStreamSynchronize(st);
     if (Ef >= 0xFFFFFFFFull) { e = cudaErrorInvalidValue; return fail("graph too large to reverse"); }
-    if ((e = grow(key, Ef * 4 + 4)) != cudaSuccess || (e = grow(val, Ef * 4 + 4)) != cudaSuccess ||
-        (e = grow(skey, Ef * 4 + 4)) != cudaSuccess || (e = grow(sval, Ef * 4 + 4)) != cudaSuccess)
+    if ((e = grow(key, Ef * 4 + 4)) != cudaSuccess || (e = grow(val, Ef * 8 + 8)) != cudaSuccess ||
+        (e = grow(skey, Ef * 4 + 4)) != cudaSuccess || (e = grow(sval, Ef * 8 + 8)) != cudaSuccess)
         return fail("alloc reverse");
     rev_edges_kernel<<<grid * 2, 256, 0, st>>>(N, ctx->offsets.as<uint64_t>(), ctx->nbr.as<uint32_t>(),
-                                               koff.as<uint64_t>(), key.as<uint32_t>(), val.as<uint32_t>(),
-                                               rc.as<uint64_t>(), ctx->errw.as<uint32_t>());
+                                               ctx->nbr_d.as<float>(), koff.as<uint64_t>(), key.as<uint32_t>(),
+                                               val.as<unsigned long long>(), ctx->errw.as<uint32_t>());
     // stable radix sort by target keeps the (i, j) order within each target
     int end_bit = 1;
     while (end_bit < 32 && (1ull << end_bit) < n) ++end_bit;
     size_t tb = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, tb, key.as<uint32_t>(), skey.as<uint32_t>(), val.as<uint32_t>(),
-                                    sval.as<uint32_t>(), (int64_t)Ef, 0, end_bit, st);
+    cub::DeviceRadixSort::SortPairs(nullptr, tb, key.as<uint32_t>(), skey.as<uint32_t>(), val.as<unsigned long long>(),
+                                    sval.as<unsigned long long>(), (int64_t)Ef, 0, end_bit, st);
     if ((e = grow(tmp, tb)) != cudaSuccess) return fail("alloc sort");
-    if ((e = cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.as<uint32_t>(), skey.as<uint32_t>(), val.as<uint32_t>(),
-                                             sval.as<uint32_t>(), (int64_t)Ef, 0, end_bit, st)) != cudaSuccess)
+    if ((e = cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.as<uint32_t>(), skey.as<uint32_t>(),
+                                             val.as<unsigned long long>(), sval.as<unsigned long long>(), (int64_t)Ef, 0,
+                                             end_bit, st)) != cudaSuccess)
         return fail("sort");
-    if ((e = scan_counts64(ctx, rc.as<uint64_t>(), toff.as<uint64_t>(), N)) != cudaSuccess) return fail("scan");
-    rev_degree_kernel<<<grid, 256, 0, st>>>(N, kcnt.as<uint64_t>(), rc.as<uint64_t>(), deg.as<uint64_t>());
-    if ((e = scan_counts64(ctx, deg.as<uint64_t>(), noff.as<uint64_t>(), N)) != cudaSuccess) return fail("scan");
+    rev_offsets_kernel<<<grid * 2, 256, 0, st>>>(N, Ef, skey.as<uint32_t>(), toff.as<uint64_t>());
+    rev_places_kernel<<<grid, 256, 0, st>>>(N, koff.as<uint64_t>(), toff.as<uint64_t>(), noff.as<uint64_t>());
     const uint64_t E2 = 2 * Ef;
     if ((e = grow(ai, E2 * 4 + 4)) != cudaSuccess || (e = grow(ad, E2 * 4 + 4)) != cudaSuccess)
         return fail("alloc reverse");
     std::cerr << "Reranking edges..." << std::endl;
-    rev_assemble_kernel<<<(N + 127) / 128, 128, 0, st>>>(
+    rev_assemble_kernel<<<ctx->num_sms * 6, REV_WARPS * 32, 0, st>>>(
         N, ctx->offsets.as<uint64_t>(), ctx->nbr.as<uint32_t>(), ctx->nbr_d.as<float>(), koff.as<uint64_t>(),
-        toff.as<uint64_t>(), sval.as<uint32_t>(), noff.as<uint64_t>(), ai.as<uint32_t>(), ad.as<float>(),
-        fdeg.as<uint64_t>());
+        toff.as<uint64_t>(), sval.as<unsigned long long>(), ai.as<uint32_t>(), ad.as<float>(), fdeg.as<uint64_t>());
     if ((e = cudaGetLastError()) != cudaSuccess) return fail("reverse");
     if ((e = scan_counts64(ctx, fdeg.as<uint64_t>(), foff.as<uint64_t>(), N)) != cudaSuccess) return fail("scan");
     uint64_t Efin = 0;

@@ -35,21 +35,6 @@ namespace kgb {
 
 namespace {
 
-template <bool HM>
-struct PoolAcc {   // accessor for gnu_sort over the smem pool (with the m|M words when HM)
-    float *d; uint32_t *i; uint32_t *m;
-    struct Rec { float d; uint32_t i, m; };
-    __device__ float key(int x) const { return d[x]; }
-    __device__ void swap(int x, int y) const {
-        float td = d[x]; d[x] = d[y]; d[y] = td;
-        uint32_t ti = i[x]; i[x] = i[y]; i[y] = ti;
-        if constexpr (HM) { uint32_t tm = m[x]; m[x] = m[y]; m[y] = tm; }
-    }
-    __device__ Rec get(int x) const { return Rec{d[x], i[x], HM ? m[x] : 0u}; }
-    __device__ void put(int x, Rec r) const { d[x] = r.d; i[x] = r.i; if constexpr (HM) m[x] = r.m; }
-    __device__ float rkey(Rec r) const { return r.d; }
-};
-
 struct WarpSmem {
     float *q;          // ld floats
     float *pd;         // cap
@@ -425,11 +410,15 @@ __global__ void __launch_bounds__(MB == 9 ? 128 : 256, MB) search_kernel(SearchA
                 __syncwarp();
             }
             // kgraph.cpp:476: std::sort by dist (GNU introsort order for ties)
-            if (lane == 0) {
-                PoolAcc<!CP> acc{s.pd, s.pid, s.pm};
-                gnu_sort(acc, 0, (int)L);
+            if (L <= (uint32_t)WARP_SORT_MAX) {
+                warp_gnu_sort(s.pd, s.pid, s.pm, (int)L, s.lid, lane);
+            } else {
+                if (lane == 0) {
+                    WarpSortAcc acc{s.pd, s.pid, s.pm};
+                    gnu_sort(acc, 0, (int)L);
+                }
+                __syncwarp();
             }
-            __syncwarp();
 
             uint32_t k = 0;
             // Each expansion advances m or clears a flag of an entry that was inserted

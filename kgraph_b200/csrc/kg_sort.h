@@ -16,8 +16,9 @@
 // sort (guarded for the first 16, unguarded after).  Comparisons are `a < b`
 // on the key only.
 //
-// Written as a template over an accessor so the same code runs in a CUDA
-// thread (device) and in the host tests that check it against std::sort.
+// gnu_sort is written as a template over an accessor so the same code runs in a CUDA
+// thread (device) and in the host tests that check it against std::sort;
+// warp_gnu_sort is the same sort by a warp.
 #pragma once
 #include <cstdint>
 
@@ -166,5 +167,138 @@ KG_HD void gnu_sort(A &a, int first, int last) {
         gs_insertion_sort(a, first, last);
     }
 }
+
+#ifdef __CUDACC__
+// gnu_sort of n <= WARP_SORT_MAX records (key d[i], payload id[i] and, unless
+// null, m[i]; shared or global memory) by one warp: the same permutation, ties
+// included.  tmp: WARP_SORT_TMP words of the warp's own shared memory.
+//  * Which ranges are partitioned, and around which pivots, depends only on the
+//    data, and ranges are disjoint, so their order is free.
+//  * A Hoare partition swaps the t-th stop of its left scan (a record not below
+//    the pivot) with the t-th stop of its right scan (one not above it) while
+//    they have not crossed; the swaps lie behind both scans.  So stops are found
+//    32 at a time, paired by rank and swapped in parallel; the cut is the next
+//    left stop, or the last right stop swapped if that comes first.
+//  * The final insertion sort is stable, and ranges that were left have at most
+//    16 records: a record's place is its own plus the smaller ones up to 15
+//    behind it minus the larger ones up to 15 before it.
+// A range whose depth limit is spent is heap-sorted by one lane.
+constexpr int WARP_SORT_MAX = 8191, WARP_SORT_TMP = 48;
+
+struct WarpSortAcc {   // the serial accessor, for the heap sort
+    float *d; uint32_t *i, *m;
+    struct Rec { float d; uint32_t i, m; };
+    __device__ float key(int x) const { return d[x]; }
+    __device__ void swap(int x, int y) const {
+        const float td = d[x]; d[x] = d[y]; d[y] = td;
+        const uint32_t ti = i[x]; i[x] = i[y]; i[y] = ti;
+        if (m) { const uint32_t tm = m[x]; m[x] = m[y]; m[y] = tm; }
+    }
+    __device__ Rec get(int x) const { return Rec{d[x], i[x], m ? m[x] : 0u}; }
+    __device__ void put(int x, Rec r) const { d[x] = r.d; i[x] = r.i; if (m) m[x] = r.m; }
+    __device__ float rkey(Rec r) const { return r.d; }
+};
+
+__device__ inline int warp_partition(float *d, uint32_t *id, uint32_t *m, int f, int l, uint8_t *rank, int lane) {
+    const unsigned ALL = 0xFFFFFFFFu, below = (1u << lane) - 1u;
+    const float piv = d[f];
+    int lp = f + 1, rp = l - 1;      // next positions to scan
+    int lb = 0, rb = 0, rlast = l;   // bases of the scanned pieces; the last right stop swapped
+    unsigned ml = 0, mr = 0;         // their stops not yet paired
+    for (;;) {
+        while (!ml) {
+            if (lp >= rlast) return rlast;
+            lb = lp;
+            const int p = lb + lane;
+            ml = __ballot_sync(ALL, p < l && !(d[p] < piv));
+            lp += 32;
+        }
+        while (!mr && rp > f) {
+            rb = rp;
+            const int p = rb - lane;
+            mr = __ballot_sync(ALL, p > f && !(piv < d[p]));
+            rp -= 32;
+        }
+        if (!mr) return min(lb + __ffs(ml) - 1, rlast);
+        const int t = min(__popc(ml), __popc(mr));
+        if ((ml >> lane) & 1u) rank[__popc(ml & below)] = (uint8_t)lane;
+        if ((mr >> lane) & 1u) rank[32 + __popc(mr & below)] = (uint8_t)lane;
+        __syncwarp();
+        int L = 0, R = 0;
+        if (lane < t) { L = lb + rank[lane]; R = rb - rank[32 + lane]; }
+        const unsigned okm = __ballot_sync(ALL, lane < t && L < R);
+        if ((okm >> lane) & 1u) {
+            const float td = d[L]; d[L] = d[R]; d[R] = td;
+            const uint32_t ti = id[L]; id[L] = id[R]; id[R] = ti;
+            if (m) { const uint32_t tm = m[L]; m[L] = m[R]; m[R] = tm; }
+        }
+        __syncwarp();
+        const int n = __popc(okm);
+        if (n) rlast = __shfl_sync(ALL, R, n - 1);
+        if (n < t) return min(__shfl_sync(ALL, L, n), rlast);
+        ml = __ballot_sync(ALL, ((ml >> lane) & 1u) && __popc(ml & below) >= t);
+        mr = __ballot_sync(ALL, ((mr >> lane) & 1u) && __popc(mr & below) >= t);
+    }
+}
+
+__device__ inline void warp_gnu_sort(float *d, uint32_t *id, uint32_t *m, int n, uint32_t *tmp, int lane) {
+    uint8_t *rank = reinterpret_cast<uint8_t *>(tmp + 32);   // 64 bytes behind 32 frames
+    int sp = 0, f = 0, l = n, depth = n > 1 ? 2 * (31 - __clz(n)) : 0;
+    for (;;) {
+        if (l - f <= 16 || depth == 0) {
+            if (l - f > 16) {
+                if (lane == 0) { WarpSortAcc a{d, id, m}; gs_heapsort(a, f, l); }
+                __syncwarp();
+            }
+            if (sp == 0) break;
+            const uint32_t w = tmp[--sp];
+            __syncwarp();
+            f = (int)(w & 8191u); l = (int)((w >> 13) & 8191u); depth = (int)(w >> 26);
+            continue;
+        }
+        --depth;
+        const int mid = f + (l - f) / 2;
+        const float a = d[f + 1], b = d[mid], c = d[l - 1];
+        int at;   // gs_move_median_to_first
+        if (a < b) at = b < c ? mid : a < c ? l - 1 : f + 1;
+        else at = a < c ? f + 1 : b < c ? l - 1 : mid;
+        __syncwarp();
+        if (lane == 0) { WarpSortAcc s{d, id, m}; s.swap(f, at); }
+        __syncwarp();
+        const int cut = warp_partition(d, id, m, f, l, rank, lane);
+        if (cut - f > 16) {
+            if (lane == 0) tmp[sp] = (uint32_t)f | (uint32_t)cut << 13 | (uint32_t)depth << 26;
+            ++sp;
+            __syncwarp();
+        }
+        f = cut;
+    }
+    // the final insertion sort; a piece of 32 is written once the next one has been ranked
+    float pd = 0.f;
+    uint32_t pi = 0, pm = 0;
+    int pp = -1;
+    for (int base = 0; base < n + 32; base += 32) {
+        const int p = base + lane;
+        float v = 0.f;
+        uint32_t vi = 0, vm = 0;
+        int np = -1;
+        if (p < n) {
+            v = d[p];
+            vi = id[p];
+            if (m) vm = m[p];
+            np = p;
+#pragma unroll 5
+            for (int o = 1; o <= 15; ++o) {
+                if (p + o < n && d[p + o] < v) ++np;
+                if (p - o >= 0 && v < d[p - o]) --np;
+            }
+        }
+        __syncwarp();
+        if (pp >= 0) { d[pp] = pd; id[pp] = pi; if (m) m[pp] = pm; }
+        __syncwarp();
+        pd = v; pi = vi; pm = vm; pp = np;
+    }
+}
+#endif
 
 }  // namespace kgb
