@@ -263,150 +263,310 @@ __global__ void __launch_bounds__(256) join_kernel(BuildState s) {
     }
 }
 
-// The same join with a node's lists staged in shared memory: one CTA per node
-// copies the rows of new ++ old (jt_rows of them; rows beyond are read from
-// global memory) and their norm terms once, then evaluates the node's pairs
-// from there -- each 4-lane group one pair per pass with the canonical
-// arithmetic (group4_raw, the same bits as pair_dist) -- so a node's partner
-// rows cross from L2/DRAM once per node instead of once per pair.  Pairs: for
-// new entry i (warp-strided), new[i+1 ..) then old, as join_kernel.
+// The same join, one CTA per node, its lists' rows staged in shared memory
+// (cp.async; jt_rows of them, the rest is read from global memory) and its pairs
+// evaluated in register tiles: a warp takes 4 new entries x 32 partners, each
+// 4-lane group 4 x 4 pairs with the canonical arithmetic (the same bits as
+// pair_dist; lane t owns canonical lanes 4t .. 4t + 3 of all 16), so a chunk of
+// 16 columns costs 8 shared-memory reads for 16 pairs a group instead of two per
+// pair.  The partial sums are reduced by exchanging halves -- lane t ends with
+// one new entry's four distances -- in the canonical tree order (addition
+// commutes).  Rows lie 16 words apart modulo 32, so the two groups of a
+// shared-memory phase read different banks.
+// Pairs: for new entry i, new[i+1 ..) then old, as join_kernel.
+// Bound: FP32 issue (a product and a sum per element, never fused) and the
+// gather of the rows.  1M x 128 mixture (64 centres), K=50 L=100 S=12: with one
+// pair per group and pass and 24 KB of rows the joins took 540 ms of a 978 ms
+// build, now 290 ms of 727.  Tried and slower: packed FP32 pairs (fewer
+// instructions at half the rate, more spills), 4 x 16 tiles for short remainders
+// (two copies of the tile code miss the instruction cache), prefetching the next
+// node's rows into L2.
 constexpr int JT_WARPS = 4;
-// Shared memory per CTA; rows past it are read from L2.  24 KB lets 8 CTAs
-// share an SM: at 1M x 128 the join runs 0.73 s a build against 0.89 s with
-// 48 KB (4 CTAs), the occupancy hiding the L2 reads of the rows left out.
-// Rows too wide for 8 of them in 24 KB take the 48 KB budget.
-#ifndef JT_SMEM_BUDGET
-#define JT_SMEM_BUDGET (24 * 1024)
-#endif
-constexpr size_t JT_SMEM_WIDE = 48 * 1024;
-constexpr uint32_t JT_BUF = 64;   // offers a warp collects before it appends them to the record buffer
+constexpr uint32_t JT_CLAIM = 8;   // nodes a CTA claims at a time
+constexpr uint32_t JT_I = 4, JT_J = 32;   // new entries x partners per warp tile
+// Shared memory per CTA: four CTAs an SM, as many as the tile's 128 registers allow.
+constexpr size_t JT_SMEM_BUDGET = 56 * 1024;
+constexpr uint32_t JT_BUF = 2 * JT_I * JT_J;   // offers a warp collects before it appends them: a tile's most
 // Shared memory of join_tile_kernel besides the rows: per list entry its id,
 // norm term and radius, per warp the offer buffer.
 __host__ __device__ constexpr size_t jt_fixed_bytes(uint32_t list_cap) {
-    return (size_t)list_cap * 12 + (size_t)JT_WARPS * JT_BUF * 16;
+    return (size_t)list_cap * 12 + (size_t)JT_WARPS * JT_BUF * 8;
 }
+__host__ __device__ constexpr uint32_t jt_stride(uint32_t ld) { return ld % 32 == 0 ? ld + 16 : ld; }   // ld: a multiple of 16
 
-// Deferred mode: the offers a warp collected (all of the CTA's current node)
-// go to the record buffer with one cursor atomic; those beyond its capacity
-// are inserted under the lock here (their uu counts for the current node).
-__device__ __forceinline__ void jt_flush(const BuildState &s, uint4 *buf, uint32_t &cnt, int lane, bool &uu,
-                                         InsertTally &tally) {
-    if (!cnt) return;
+// Deferred mode: the offers a warp collected (all of the CTA's current node:
+// target and candidate as list positions, the distance) go to the record buffer
+// with one cursor atomic; those beyond its capacity are inserted under the lock
+// here.  Returns whether such an x <- y insert landed below K.  Out of line: the
+// tile code it is called from must stay within the instruction cache.
+constexpr uint32_t JT_UU = 1u << 30;   // the pair's x <- y offer
+__device__ __noinline__ bool jt_flush(const BuildState &s, const uint2 *buf, const uint32_t *uid, uint32_t n,
+                                      uint32_t cnt, int lane) {
     unsigned long long b0 = 0;
     if (lane == 0) b0 = atomicAdd(s.off_cursor, (unsigned long long)cnt);
     b0 = __shfl_sync(FULL, b0, 0);
     const uint32_t fit = b0 >= s.off_cap ? 0u : (uint32_t)min((unsigned long long)cnt, s.off_cap - b0);
     for (uint32_t k = lane; k < fit; k += 32) {
-        const uint4 o = buf[k];
-        s.off_lin[b0 + k] = o;
-        atomicAdd(s.off_cnt + o.x, 1u);
+        const uint2 o = buf[k];
+        const uint32_t tg = uid[o.x & 0x7FFFu];
+        s.off_lin[b0 + k] = make_uint4(tg, uid[(o.x >> 15) & 0x7FFFu], o.y, n | ((o.x & JT_UU) ? OFFER_UU : 0u));
+        atomicAdd(s.off_cnt + tg, 1u);
     }
-    for (uint32_t k = fit; k < cnt; ++k) {
-        const uint4 o = buf[k];
-        const uint32_t r = locked_insert(s, o.x, o.y, __uint_as_float(o.z), lane, tally);
-        if ((o.w & OFFER_UU) && r < s.K) uu = true;
+    bool uu = false;
+    if (fit < cnt) {
+        InsertTally tally;
+        for (uint32_t k = fit; k < cnt; ++k) {
+            const uint2 o = buf[k];
+            const uint32_t r =
+                locked_insert(s, uid[o.x & 0x7FFFu], uid[(o.x >> 15) & 0x7FFFu], __uint_as_float(o.y), lane, tally);
+            if ((o.x & JT_UU) && r < s.K) uu = true;
+        }
+        if (lane == 0) {
+            atomicAdd(s.inserts, tally.attempts);
+            atomicAdd(s.inserts + 1, tally.landed);
+        }
     }
-    cnt = 0;
     __syncwarp();
+    return uu;
 }
 
-__global__ void __launch_bounds__(JT_WARPS * 32) join_tile_kernel(BuildState s) {
+// One row chunk's 4 x 4 products of a lane.
+template <bool L2>
+__device__ __forceinline__ void jt_acc(float4 &acc, const float4 &x, const float4 &y) {
+    lane_acc(acc, x, y, L2 ? METRIC_L2SQR : METRIC_EUCLIDEAN);
+}
+
+// Canonical raw sums of the tile's pairs: pi[k] / pj[k] point at this lane's
+// part of rows k.  Returns in v[k] the pair (new entry 2 (t & 1) + (t >> 1),
+// partner k of this group).
+template <bool L2>
+__device__ __forceinline__ void jt_reduce(float4 (&acc)[4][4], int t, float (&v)[4]) {
+    const bool o1 = t & 1, o2 = t & 2;
+    float4 r[2][4];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 keep = o1 ? acc[2 + k][j] : acc[k][j], send = o1 ? acc[k][j] : acc[2 + k][j];
+            r[k][j].x = __fadd_rn(keep.x, __shfl_xor_sync(FULL, send.x, 1));
+            r[k][j].y = __fadd_rn(keep.y, __shfl_xor_sync(FULL, send.y, 1));
+            r[k][j].z = __fadd_rn(keep.z, __shfl_xor_sync(FULL, send.z, 1));
+            r[k][j].w = __fadd_rn(keep.w, __shfl_xor_sync(FULL, send.w, 1));
+        }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float4 keep = o2 ? r[1][j] : r[0][j], send = o2 ? r[0][j] : r[1][j];
+        const float x = __fadd_rn(keep.x, __shfl_xor_sync(FULL, send.x, 2));
+        const float y = __fadd_rn(keep.y, __shfl_xor_sync(FULL, send.y, 2));
+        const float z = __fadd_rn(keep.z, __shfl_xor_sync(FULL, send.z, 2));
+        const float w = __fadd_rn(keep.w, __shfl_xor_sync(FULL, send.w, 2));
+        v[j] = __fadd_rn(__fadd_rn(x, y), __fadd_rn(z, w));
+    }
+}
+
+// The tail elements of a pair's canonical sum (as group4_raw).
+template <bool L2>
+__device__ __forceinline__ float jt_tail(float r, const float *a, const float *b, int d) {
+    int i = d & ~15;
+    if (d - i >= 8) {
+        for (int e = i + 8; i < e; ++i) {
+            float x = a[i], y = b[i];
+            if (L2) { x = __fsub_rn(x, y); y = x; }
+            r = __fadd_rn(r, __fmul_rn(x, y));
+        }
+    }
+    for (; i < d; ++i) {
+        float x = a[i], y = b[i];
+        if (L2) { x = __fsub_rn(x, y); y = x; }
+        r = __fmaf_rn(x, y, r);
+    }
+    return r;
+}
+
+template <bool L2>
+__global__ void __launch_bounds__(JT_WARPS * 32, 4) join_tile_kernel(const __grid_constant__ BuildState s) {
     extern __shared__ __align__(16) float jt_smem[];
-    __shared__ uint32_t s_node, s_uu;
+    __shared__ uint32_t s_cnt, s_uu, s_list[JT_CLAIM], s_a[JT_CLAIM], s_b[JT_CLAIM];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const uint32_t N = s.D.n, stride = s.D.ld + 4;   // 16 bytes of padding: rows start on different banks
-    const int metric = s.D.metric;
-    const uint32_t cap = s.NEWCAP + s.OLDCAP;
-    uint4 *bufs = reinterpret_cast<uint4 *>(jt_smem);   // 16-byte aligned at the start
-    uint4 *buf = bufs + (size_t)warp * JT_BUF;
-    float *rows = reinterpret_cast<float *>(bufs + (size_t)JT_WARPS * JT_BUF);
-    float *nrm = rows + (size_t)s.jt_rows * stride;
+    const uint32_t N = s.D.n, ld = s.D.ld, stride = jt_stride(ld), cap = s.NEWCAP + s.OLDCAP;
+    const int chunks = (int)s.D.d >> 4, metric = s.D.metric;
+    float *rows = jt_smem;   // 16-byte aligned, rows of 64-byte multiples
+    uint2 *buf = reinterpret_cast<uint2 *>(rows + (size_t)s.jt_rows * stride) + (size_t)warp * JT_BUF;
+    float *nrm = reinterpret_cast<float *>(reinterpret_cast<uint2 *>(rows + (size_t)s.jt_rows * stride) + JT_WARPS * JT_BUF);
     float *rad = nrm + cap;
     uint32_t *uid = reinterpret_cast<uint32_t *>(rad + cap);
-    const bool deferred = s.off_lin != nullptr;
-    unsigned long long comps = 0;
-    InsertTally tally;
-    uint32_t bcnt = 0;
+    unsigned long long comps = 0;   // per lane
+    uint32_t bcnt = 0, next = 0;
+    if (threadIdx.x == 0) next = s.node_lo + atomicAdd(s.work, JT_CLAIM);
+    uint32_t li = 0, cnt = 0;
     for (;;) {
-        if (threadIdx.x == 0) { s_node = s.node_lo + atomicAdd(s.work, 1u); s_uu = 0; }
-        __syncthreads();
-        const uint32_t n = s_node;
-        if (n >= s.node_hi) break;
-        const uint32_t a = min(s.cnt_new[n], s.NEWCAP), b = min(s.cnt_old[n], s.OLDCAP);
-        if (a == 0) {
-            if (threadIdx.x == 0) s.found[n] = 0u;
+        if (li == cnt) {   // the next run of nodes; those without new entries have no pairs
+            if (warp == 0) {
+                const uint32_t base = __shfl_sync(FULL, next, 0), x = base + lane;
+                const bool in = lane < (int)JT_CLAIM && x < s.node_hi;
+                const uint32_t ca = in ? min(s.cnt_new[x], s.NEWCAP) : 0u, cb = in ? min(s.cnt_old[x], s.OLDCAP) : 0u;
+                if (in && !ca) s.found[x] = 0u;
+                const unsigned am = __ballot_sync(FULL, ca > 0);
+                if (ca) {
+                    const int at = __popc(am & ((1u << lane) - 1u));
+                    s_list[at] = x;
+                    s_a[at] = ca;
+                    s_b[at] = cb;
+                }
+                if (lane == 0) {
+                    s_cnt = base < s.node_hi ? __popc(am) : NO_ID;
+                    if (base < s.node_hi) next = s.node_lo + atomicAdd(s.work, JT_CLAIM);   // needed when this run is done
+                    s_uu = 0;
+                }
+            }
             __syncthreads();
-            continue;
+            cnt = s_cnt;
+            li = 0;
+            if (cnt == NO_ID) break;
+            if (cnt == 0) { __syncthreads(); continue; }
         }
-        const uint32_t U = a + b;
+        const uint32_t n = s_list[li], a = s_a[li], b = s_b[li];
+        ++li;
+        const uint32_t U = a + b, staged = min(U, s.jt_rows);
         const uint32_t *nw = s.nn_new + (size_t)n * s.NEWCAP, *od = s.nn_old + (size_t)n * s.OLDCAP;
         for (uint32_t u = threadIdx.x; u < U; u += blockDim.x) {
             uint32_t id = u < a ? nw[u] : od[u - a];
             if (id >= N) { raise_error(s.err, ERR_BAD_ID); id = NO_ID; }
             uid[u] = id;
-            nrm[u] = (id != NO_ID && metric != METRIC_L2SQR) ? s.D.norms[id] : 0.f;
-            // deferred: the radii as the join starts (they change only in the merge after it; a
-            // larger radius lets more offers through to the merge's exact test)
-            rad[u] = id != NO_ID ? *reinterpret_cast<volatile float *>(s.radius + id) : 0.f;
         }
         __syncthreads();
-        const uint32_t staged = min(U, s.jt_rows);
         for (uint32_t r = warp; r < staged; r += JT_WARPS) {
             const uint32_t id = uid[r] == NO_ID ? 0u : uid[r];
-            const float *src = s.D.X + (size_t)id * s.D.ld;
-            float *dst = rows + (size_t)r * stride;
-            for (uint32_t k = 4 * lane; k < s.D.ld; k += 128) *reinterpret_cast<float4 *>(dst + k) = ld4(src + k);
+            const float *src = s.D.X + (size_t)id * ld;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(rows + (size_t)r * stride);
+            for (uint32_t k = 4 * lane; k < ld; k += 128)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 4 * k), "l"(src + k) : "memory");
         }
+        for (uint32_t u = threadIdx.x; u < U; u += blockDim.x) {
+            const uint32_t id = uid[u];
+            nrm[u] = (id != NO_ID && !L2) ? s.D.norms[id] : 0.f;
+            // the radii as the join starts (they change only in the merge after it; a larger radius
+            // lets more offers through to the merge's exact test)
+            rad[u] = id != NO_ID ? *reinterpret_cast<volatile float *>(s.radius + id) : 0.f;
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
         bool uu = false;
-        for (uint32_t i = warp; i < a; i += JT_WARPS) {
-            const uint32_t idi = uid[i];
-            const float *ri = i < s.jt_rows ? rows + (size_t)i * stride : s.D.X + (size_t)(idi == NO_ID ? 0u : idi) * s.D.ld;
-            const float ni = nrm[i], radi = rad[i];
-            const uint32_t nnn = a - 1 - i, inner = nnn + b;   // partners: new[i+1..a) then old
-            for (uint32_t base = 0; base < inner; base += 8) {
-                const uint32_t k = base + g;
-                const bool in = k < inner;
-                const uint32_t u = in ? (k < nnn ? i + 1 + k : a + (k - nnn)) : i;
-                const bool is_nn = u < a;
-                const uint32_t jid = uid[u];
-                // i < j by id excludes equal ids among the new entries (kgraph.cpp:742-743)
-                const bool v = in && idi != NO_ID && jid != NO_ID && !(is_nn && jid == idi);
-                const float *rj = u < s.jt_rows ? rows + (size_t)u * stride : s.D.X + (size_t)(jid == NO_ID ? 0u : jid) * s.D.ld;
-                const float raw = group4_raw(ri, rj, (int)s.D.d, metric, t, FULL);
-                const float dd = metric == METRIC_L2SQR ? raw : finish_metric(raw, ni, nrm[u], metric);
-                const bool i_is_x = !is_nn || idi < jid;
-                const uint32_t x = v ? (i_is_x ? idi : jid) : 0u, y = v ? (i_is_x ? jid : idi) : 0u;
-                if (!deferred) {
-                    settle_pass(s, lane, t, v, x, y, dd, n, comps, uu, tally);
-                    continue;
+        uint32_t tile = 0;   // tiles of this node, dealt to the warps in turn
+        for (uint32_t ib = 0; ib < a; ib += JT_I)
+            for (uint32_t jb = ib + 1; jb < U; jb += JT_J, ++tile) {
+                if (tile % JT_WARPS != (uint32_t)warp) continue;
+                float4 acc[4][4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                const float *ri, *rj[4];   // this lane's new entry (after the reduction) and partners, for the tail
+                const uint32_t mi = ib + 2 * (t & 1) + (t >> 1);
+                if (ib + JT_I <= s.jt_rows && jb + JT_J <= s.jt_rows) {   // rows past U: unused, masked below
+                    const float *pi = rows + (size_t)ib * stride + 4 * t, *pj = rows + (size_t)(jb + g) * stride + 4 * t;
+                    const uint32_t sj = 8 * stride;
+                    for (int c = 0; c < chunks; ++c) {
+                        float4 x[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) x[i] = ld4(pi + i * stride + 16 * c);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const float4 y = ld4(pj + j * sj + 16 * c);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) jt_acc<L2>(acc[i][j], x[i], y);
+                        }
+                    }
+                    ri = rows + (size_t)mi * stride;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) rj[j] = rows + (size_t)(jb + 8 * j + g) * stride;
+                } else {
+                    auto row = [&](uint32_t u) -> const float * {
+                        if (u < staged) return rows + (size_t)u * stride;
+                        const uint32_t id = u < U ? uid[u] : 0u;
+                        return s.D.X + (size_t)(id == NO_ID ? 0u : id) * ld;
+                    };
+                    const float *pi[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) pi[i] = row(ib + i);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) rj[j] = row(jb + 8 * j + g);
+                    ri = row(mi);
+#pragma unroll 1
+                    for (int c = 0; c < chunks; ++c) {
+                        float4 x[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) x[i] = ld4(pi[i] + 16 * c + 4 * t);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const float4 y = ld4(rj[j] + 16 * c + 4 * t);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) jt_acc<L2>(acc[i][j], x[i], y);
+                        }
+                    }
                 }
-                // the unlocked radius test of both directions (kgraph.cpp:725) on the staged radii
-                const float rx = i_is_x ? radi : rad[u], ry = i_is_x ? rad[u] : radi;
-                comps += __popc(__ballot_sync(FULL, v && t == 0));
-                const bool off = v && ((t == 0 && !(dd > rx)) || (t == 1 && !(dd > ry)));
-                const unsigned om = __ballot_sync(FULL, off);
-                if (!om) continue;
-                if (bcnt + __popc(om) > JT_BUF) jt_flush(s, buf, bcnt, lane, uu, tally);
-                if (off) {
-                    const uint32_t pos = bcnt + __popc(om & ((1u << lane) - 1u));
-                    buf[pos] = make_uint4(t == 0 ? x : y, t == 0 ? y : x, __float_as_uint(dd), n | (t == 0 ? OFFER_UU : 0u));
+                float v[4];
+                jt_reduce<L2>(acc, t, v);
+                // this lane: new entry mi against partners jb + 8 j + g
+                const bool iok = mi < a;
+                const uint32_t idi = iok ? uid[mi] : NO_ID;
+                const float ni = iok ? nrm[mi] : 0.f, radi = iok ? rad[mi] : 0.f;
+                uint32_t offers = 0;   // bit 2j: to the new entry, 2j + 1: to the partner
+                uint32_t xbit = 0;     // bit j: the new entry is the pair's x
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t u = jb + 8 * j + g;
+                    if (idi == NO_ID || u >= U || u <= mi) continue;
+                    const uint32_t jid = uid[u];
+                    const bool is_nn = u < a;
+                    // i < j by id excludes equal ids among the new entries (kgraph.cpp:742-743)
+                    if (jid == NO_ID || (is_nn && jid == idi)) continue;
+                    ++comps;
+                    float raw = v[j];
+                    if (s.D.d & 15u) raw = jt_tail<L2>(raw, ri, rj[j], (int)s.D.d);
+                    const float dd = L2 ? raw : finish_metric(raw, ni, nrm[u], metric);
+                    v[j] = dd;
+                    if (!is_nn || idi < jid) xbit |= 1u << j;
+                    // the unlocked radius test of both directions (kgraph.cpp:725) on the staged radii
+                    if (!(dd > radi)) offers |= 1u << (2 * j);
+                    if (!(dd > rad[u])) offers |= 2u << (2 * j);
                 }
-                bcnt += __popc(om);
+                const uint32_t mine = __popc(offers);
+                uint32_t end = mine;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t w = __shfl_up_sync(FULL, end, o);
+                    if (lane >= o) end += w;
+                }
+                const uint32_t total = __shfl_sync(FULL, end, 31);
+                if (!total) continue;
+                if (bcnt + total > JT_BUF) {
+                    uu |= jt_flush(s, buf, uid, n, bcnt, lane);
+                    bcnt = 0;
+                }
+                uint32_t at = bcnt + end - mine;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t u = jb + 8 * j + g, ix = (xbit >> j) & 1u;
+                    if (offers & (1u << (2 * j))) buf[at++] = make_uint2(mi | u << 15 | (ix ? JT_UU : 0u), __float_as_uint(v[j]));
+                    if (offers & (2u << (2 * j))) buf[at++] = make_uint2(u | mi << 15 | (ix ? 0u : JT_UU), __float_as_uint(v[j]));
+                }
+                bcnt += total;
                 __syncwarp();
             }
+        if (bcnt) {
+            uu |= jt_flush(s, buf, uid, n, bcnt, lane);
+            bcnt = 0;
         }
-        if (deferred) jt_flush(s, buf, bcnt, lane, uu, tally);
         if (uu && lane == 0) atomicOr(&s_uu, 1u);
         __syncthreads();
-        if (threadIdx.x == 0) s.found[n] = s_uu;
+        if (threadIdx.x == 0) {
+            s.found[n] = s_uu;
+            s_uu = 0;
+        }
     }
+    for (int o = 16; o; o >>= 1) comps += __shfl_xor_sync(FULL, comps, o);
     if (lane == 0 && comps) atomicAdd(s.n_comps, comps);
-    if (lane == 0 && tally.attempts) {
-        atomicAdd(s.inserts, tally.attempts);
-        atomicAdd(s.inserts + 1, tally.landed);
-    }
 }
 
 // ------------------------------------------------------------------ deferred inserts
@@ -1217,13 +1377,16 @@ extern "C" int kg_build(kg_ctx *ctx, const kg_index_params *params, kg_index_inf
     // same pools' locks)
     if (ctx->join_tile && ctx->join_inserts != KG_INSERTS_LOCKED) {
         const size_t fixed = jt_fixed_bytes(s.NEWCAP + s.OLDCAP);
-        const size_t row_bytes = (size_t)(s.D.ld + 4) * 4;
-        size_t budget = (size_t)JT_SMEM_BUDGET - 64;
-        if (budget <= fixed + 8 * row_bytes) budget = JT_SMEM_WIDE - 64;
+        const size_t row_bytes = (size_t)jt_stride(s.D.ld) * 4, budget = JT_SMEM_BUDGET - 64;
         if (budget > fixed + 8 * row_bytes) {
-            s.jt_rows = (uint32_t)std::min<size_t>((budget - fixed) / row_bytes, s.NEWCAP + s.OLDCAP);
+            // (whole tiles of partners past the longest list can be read from shared memory)
+            s.jt_rows = (uint32_t)std::min<size_t>((budget - fixed) / row_bytes, s.NEWCAP + s.OLDCAP + JT_J);
             jt_smem = fixed + (size_t)s.jt_rows * row_bytes;
-            jt_blocks = (int)std::min<size_t>(8, (228u << 10) / (jt_smem + 1024));   // CTAs per SM it allows
+            jt_blocks = (int)std::min<size_t>(4, (228u << 10) / (jt_smem + 1024));   // CTAs per SM it allows
+            const void *fn = s.D.metric == METRIC_L2SQR ? (const void *)join_tile_kernel<true> : (const void *)join_tile_kernel<false>;
+            if (jt_smem > 48 * 1024 &&
+                (e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jt_smem)) != cudaSuccess)
+                return cuda_fail(ctx, e, "join");
         }
     }
     // Deferred inserts of the FP32 join: the offer records (linear and grouped,
@@ -1349,8 +1512,10 @@ extern "C" int kg_build(kg_ctx *ctx, const kg_index_params *params, kg_index_inf
             sr.node_hi = (uint32_t)((uint64_t)N * (r + 1) / join_rounds);
             cudaMemsetAsync(s.work, 0, 4, st);
             if (s.off_lin) rec_offers_begin();
-            if (s.jt_rows)
-                join_tile_kernel<<<ctx->num_sms * jt_blocks, JT_WARPS * 32, jt_smem, st>>>(sr);
+            if (s.jt_rows && s.D.metric == METRIC_L2SQR)
+                join_tile_kernel<true><<<ctx->num_sms * jt_blocks, JT_WARPS * 32, jt_smem, st>>>(sr);
+            else if (s.jt_rows)
+                join_tile_kernel<false><<<ctx->num_sms * jt_blocks, JT_WARPS * 32, jt_smem, st>>>(sr);
             else
                 join_kernel<<<grid_for(ctx), 256, 0, st>>>(sr);
             if (s.off_lin) {
