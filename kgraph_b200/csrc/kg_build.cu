@@ -590,43 +590,61 @@ __device__ __forceinline__ float ord2f(uint32_t u) { return __uint_as_float((u &
 
 // Ascending bitonic sort of the 32 E keys at keys[0, 32 E) by one warp, in
 // registers: lane l holds elements l E .. l E + E - 1, so partners closer than
-// E are in the lane and farther ones are an XOR shuffle away.
+// E are in the lane and farther ones are an XOR shuffle away.  The stages loop
+// over one copy of the lane's merge and of the shuffle step: unrolled, the sort
+// alone was more code than the instruction cache holds, and each warp fetched it
+// once per pool (7.7 of 16 stall cycles per issue were instruction fetches).  With
+// at most 256 keys a pass the merge also needs half the registers (100 -> 48) and
+// shared memory.  1M x 128 mixture, whole build 727 -> 606 ms.
+template <int E>
+__device__ __forceinline__ void lane_merge(unsigned long long (&v)[E], bool asc) {   // bitonic in the lane -> sorted
+#pragma unroll
+    for (int j = E / 2; j > 0; j >>= 1)
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            if (e & j) continue;
+            const unsigned long long a = v[e], b = v[e | j];
+            if ((a > b) == asc) { v[e] = b; v[e | j] = a; }
+        }
+}
 template <int E>
 __device__ __forceinline__ void warp_sort_keys(unsigned long long *keys, int lane) {
     unsigned long long v[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) v[e] = keys[lane * E + e];
+    // each lane's E keys, ascending in even lanes
 #pragma unroll
-    for (int k = 2; k <= 32 * E; k <<= 1) {
+    for (int k = 2; k <= E; k <<= 1)
 #pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                if (e & j) continue;
+                const bool asc = k < E ? (e & k) == 0 : (lane & 1) == 0;
+                const unsigned long long a = v[e], b = v[e | j];
+                if ((a > b) == asc) { v[e] = b; v[e | j] = a; }
+            }
+#pragma unroll 1
+    for (int k = 2; k <= 32; k <<= 1) {   // runs of k lanes
+        const bool asc = (lane & k) == 0;
+#pragma unroll 1
         for (int j = k >> 1; j > 0; j >>= 1) {
-            if (j >= E) {
-                const int lj = j / E;
-                const bool lower = (lane & lj) == 0;
+            const bool low = ((lane & j) == 0) == asc;
 #pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    const unsigned long long o = __shfl_xor_sync(FULL, v[e], lj);
-                    const bool asc = ((lane * E + e) & k) == 0;
-                    v[e] = (lower == asc) ? (v[e] < o ? v[e] : o) : (v[e] > o ? v[e] : o);
-                }
-            } else {
-#pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    if (e & j) continue;
-                    const bool asc = ((lane * E + e) & k) == 0;
-                    const unsigned long long a = v[e], b = v[e | j];
-                    if ((a > b) == asc) { v[e] = b; v[e | j] = a; }
-                }
+            for (int e = 0; e < E; ++e) {
+                const unsigned long long o = __shfl_xor_sync(FULL, v[e], j);
+                if ((v[e] < o) != low) v[e] = o;
             }
         }
+        lane_merge<E>(v, asc);
     }
 #pragma unroll
     for (int e = 0; e < E; ++e) keys[lane * E + e] = v[e];
     __syncwarp();
 }
 
-constexpr uint32_t MG_CH = 512;     // offers merged per pass at most (sorted in shared memory)
-constexpr uint32_t MG_PASS = 224;   // offers a value-mode pass aims at
+constexpr uint32_t MG_CH = 256;     // offers merged per pass at most (sorted in shared memory)
+constexpr uint32_t MG_PASS = 160;   // offers a value-mode pass aims at where they do not all fit
 constexpr int MG_WARPS = 8;
 size_t merge_warp_bytes(uint32_t PS) { return (size_t)MG_CH * 20 + (size_t)PS * 16; }
 
@@ -766,7 +784,7 @@ __global__ void __launch_bounds__(MG_WARPS * 32) offer_merge_kernel(BuildState s
                 uint32_t hi_key = 0xFFFFFFFFu;
                 int idx = -1;
                 uint32_t sk = 0xFFFFFFFFu;
-                if (rem > MG_PASS) {
+                if (rem > MG_CH) {
                     const uint32_t si = (uint32_t)(((uint64_t)lane * m) >> 5);
                     const uint32_t so = f2ord(__uint_as_float(s.off_grp[o0 + si].z));
                     const bool valid = !have_lo || so > lo_key;
@@ -840,8 +858,7 @@ __global__ void __launch_bounds__(MG_WARPS * 32) offer_merge_kernel(BuildState s
                 case 32: warp_sort_keys<1>(keys, lane); break;
                 case 64: warp_sort_keys<2>(keys, lane); break;
                 case 128: warp_sort_keys<4>(keys, lane); break;
-                case 256: warp_sort_keys<8>(keys, lane); break;
-                default: warp_sort_keys<16>(keys, lane); break;
+                default: warp_sort_keys<8>(keys, lane); break;
             }
             // positions of the non-duplicates
             uint32_t nnd = 0;
