@@ -534,6 +534,7 @@ __global__ void __launch_bounds__(MB == 9 ? 128 : 256, MB) search_kernel(SearchA
                     const uint32_t n = __popc(__ballot_sync(FULL, act));   // act is a prefix of the lanes
                     if (n == 0) break;   // moved, and the rest lies behind the batch
                     const uint32_t *list = s.lid + lb;
+                    const bool again = lb > 0;   // the window's second group or later
                     lb += n;
                     // an id that recurs in the group: its first position only, as the reference's
                     // in-order loop marks it visited there (kgraph.cpp:497-498)
@@ -548,13 +549,19 @@ __global__ void __launch_bounds__(MB == 9 ? 128 : 256, MB) search_kernel(SearchA
                             else prefetch_row(a.D, pid2);
                         }
                     }
-                    // All in flight together: the exact test-and-set of the visited bit, the
-                    // candidate's {M, degree}, and its row (distance).
-                    bool isnew = false;
+                    // FP32 walk: the exact test-and-set of the visited bits in flight with the
+                    // candidates' {M, degree} and rows.  Filtered walk: most candidates end with
+                    // their compressed rows, which are there before a test-and-set would be; a
+                    // candidate is new unless its id came up in an earlier group of the window,
+                    // and is marked once the batches that are taken are known (10k queries on
+                    // 200k x 100, angular, P=700: 82 -> 65 ms).
+                    constexpr bool EARLY = PREC == 0;
+                    bool isnew = cand;
                     uint32_t aM = 0;
                     if (cand) {
                         const uint32_t bit = 1u << (id & 31);
-                        isnew = !(atomicOr(vis + (id >> 5), bit) & bit);
+                        if (EARLY) isnew = !(atomicOr(vis + (id >> 5), bit) & bit);
+                        else if (again) isnew = !(__ldcg(vis + (id >> 5)) & bit);
                     }
                     float dd = 0.f;
                     unsigned nm, im, sm = 0;   // new candidates; those that may enter the pool; those skipped
@@ -612,7 +619,7 @@ __global__ void __launch_bounds__(MB == 9 ? 128 : 256, MB) search_kernel(SearchA
                                 }
                             }
                             taken = __ballot_sync(FULL, b <= bs);
-                            if (isnew && b > bs) atomicAnd(vis + (id >> 5), ~(1u << (id & 31)));
+                            if (EARLY && isnew && b > bs) atomicAnd(vis + (id >> 5), ~(1u << (id & 31)));
                             if (im & ~taken) {
                                 im &= taken;
                                 f = warp_rank_again(im, dd, lane);
@@ -623,6 +630,10 @@ __global__ void __launch_bounds__(MB == 9 ? 128 : 256, MB) search_kernel(SearchA
                         L = warp_apply_batch(s.pd, s.pid, CP ? nullptr : s.pm, L, cap, im, ai, f, dd, id | FLAG_BIT,
                                              aM << 16, lane);   // new entries: flag set, m = 0, M = actual_M
                         if (mr < k) k = mr;
+                    }
+                    if (!EARLY) {
+                        if (((nm & taken) >> lane) & 1u) atomicOr(vis + (id >> 5), 1u << (id & 31));
+                        __syncwarp();   // the bits before the next look at them
                     }
                     n_comps += __popc(nm & taken);
                     if (PREC && full) {
