@@ -129,7 +129,8 @@ int kg_search_batch(kg_ctx *ctx, const float *queries, size_t nq, size_t q_strid
  *                    node's min(max(M, params M), degree) <= (2^(31 - id
  *                    bits) - 1) S); elsewhere the 12-byte entry runs.
  *                    A new context starts with split 4, warps_per_block 0,
- *                    prefetch 2, regs 64, compact 1.
+ *                    prefetch 2, regs 64, compact 1; until a shape is set or
+ *                    tuned, a search on narrow rows takes split 2.
  * ms / default_ms / variants are filled by kg_search_autotune. */
 typedef struct {
     unsigned split, warps_per_block, prefetch;

@@ -321,7 +321,7 @@ namespace kgb {
 // instead of from `ids`.
 int search_locked(kg_ctx *ctx, const float *queries, size_t nq, size_t q_stride_bytes,
                   const kg_search_params *params, const uint32_t *K_per_q, const uint32_t *P_per_q, size_t out_ld,
-                  uint32_t *ids, float *dists, uint32_t *counts, float *costs, const SearchShape &sh,
+                  uint32_t *ids, float *dists, uint32_t *counts, float *costs, const SearchShape &shape,
                   const uint32_t *init_dev, size_t init_ld) {
     if (!ctx->has_data) return set_error(ctx, KG_E_RUNTIME, "no dataset");
     if (!params || !ids || !counts) return set_error(ctx, KG_E_INVALID, "bad arguments");
@@ -492,6 +492,8 @@ int search_locked(kg_ctx *ctx, const float *queries, size_t nq, size_t q_stride_
         a.Xc = ctx->Xc.p;
         a.cmeta = ctx->cmeta.as<float4>();
     }
+    SearchShape sh = shape;
+    if (sh.free_split) sh.split = search_split(ctx->d, ld, a.prec, Q, ctx->num_sms);
     // visited sets: one per resident warp
     a.vwords = ((N + 31) / 32 + 3) / 4 * 4;
     uint32_t slots = search_max_slots(a, sh, ctx->num_sms);
@@ -671,6 +673,8 @@ int kg_search_autotune(kg_ctx *ctx, const float *queries, size_t nq, size_t q_st
     if (r != KG_OK) return r;
     ref_ids = ids; ref_d = dists; ref_n = counts; ref_c = costs;
     top_ms = def_ms;
+    top.split = ctx->last_shape.split;   // what ran, where the batch chose its split
+    top.free_split = false;
     ++variants;
     // the 80-register budget only has FP32-walk variants
     const std::vector<uint32_t> budgets =

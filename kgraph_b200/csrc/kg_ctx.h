@@ -78,7 +78,7 @@ struct kg_ctx {
     kgb::DevBuf ell, meta;
     uint32_t ell_w = 0;
     uint32_t max_degree = 0, max_mdeg = 0;   // largest degree and largest min(M, degree) of the graph
-    kgb::SearchShape search_shape;   // launch shape of the search kernel (kg_search_autotune)
+    kgb::SearchShape search_shape{4, 0, 2, 64, 1, true};   // launch shape of the search kernel (kg_search_autotune)
     kgb::SearchShape last_shape;     // the shape the last kg_search_batch launched (kg_last_search_shape)
     uint64_t layout_version = ~0ull;
 

@@ -737,6 +737,22 @@ cudaError_t launch_filter_bounds(const SearchArgs &a, const uint32_t *ids, uint3
     return cudaGetLastError();
 }
 
+// Two lanes per distance put 16 candidates in a pass instead of 8: half the
+// passes, each a memory round trip, for twice the loads per lane.  That wins
+// where a row is few chunks of 16 columns (or ends in a tail, which every lane of
+// a group adds up by itself).  Measured on 60k uniform and 300k mixture rows, 2 /
+// 1,000 / 30,000 queries, 4 lanes against 2: FP32 d = 12 to 60 1.00-1.36x, d = 64
+// 0.94-1.07x, d = 96 0.90-1.05x; BF16 filter d = 12 to 96 0.99-1.29x; FP8 filter
+// (whose row chunk is 4 bytes a lane) d <= 26 1.07-1.22x, above it 1.01-1.27x for
+// up to 1,000 queries and 0.91-0.99x for 30,000.
+uint32_t search_split(uint32_t d, uint32_t ld, uint32_t prec, size_t nq, int num_sms) {
+    bool two;
+    if (prec == 0) two = d < 64;
+    else if (prec == 1) two = ld <= 96;
+    else two = d < 32 || (ld <= 96 && nq <= (size_t)num_sms * 8);
+    return two ? 2 : 4;
+}
+
 size_t search_warp_smem_bytes(uint32_t ld, uint32_t cap, uint32_t rcap, bool compact) {
     size_t b = sizeof(float) * ld + (compact ? 8ull : 12ull) * cap + 8ull * rcap + 12ull * 32;
     return (b + 15) & ~size_t(15);

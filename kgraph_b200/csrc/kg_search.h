@@ -52,7 +52,11 @@ struct SearchArgs {
 // where SearchArgs::compact_ok).  Every shape computes the same bits.
 struct SearchShape {
     uint32_t split = 4, warps_per_block = 0, prefetch = 2, regs = 64, compact = 1;
+    bool free_split = false;   // a context's shape before anyone chose one: search_split picks the D-split
 };
+// The D-split of a batch of nq queries on rows of d (padded ld) columns where
+// the caller has not chosen one (prec: the filter's rows, 0 none).
+uint32_t search_split(uint32_t d, uint32_t ld, uint32_t prec, size_t nq, int num_sms);
 bool search_shape_valid(const SearchShape &sh);
 // Whether a launch of shape sh with arguments a runs the compact pool entry.
 bool search_uses_compact(const SearchArgs &a, const SearchShape &sh);
