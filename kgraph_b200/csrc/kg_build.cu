@@ -569,6 +569,218 @@ __global__ void __launch_bounds__(JT_WARPS * 32, 4) join_tile_kernel(const __gri
     if (lane == 0 && comps) atomicAdd(s.n_comps, comps);
 }
 
+// The same join for narrow rows (ld <= JL_MAX_LD): one warp per node and one pair
+// per lane.  A lane keeps one partner's row in registers and meets the new
+// entries one after the other, read from shared memory as broadcasts, so the
+// canonical 16 partial sums and their tree stay in the lane: a pair of 16 columns
+// is 31 instructions, where the 4-lane groups above spend two thirds of theirs on
+// exchanging partial sums and dealing tiles.  Warps share nothing, so none waits
+// for another's tiles, and a warp's loads hide behind the other warps' pairs.
+// Bound: FP32 and shared-memory issue (a broadcast 16-byte read costs four
+// cycles of the shared-memory pipe, an eighth of the pairs' FP32 instructions it
+// feeds): beyond 64 columns the tiles' reuse wins.  Whole builds, tiles against
+// this: 100k x 16 uniform 22.5 -> 17.1 ms, 100k x 26 32.9 -> 22.4, 200k x 48
+// mixture (K=50 L=100 S=12) 57.6 -> 45.0, 200k x 64 59.6 -> 51.2, 100k x 64
+// angular 51.0 -> 37.4.  Two partners a lane only at 16 columns: at 32 they cost
+// a fifth of the warps (22.4 -> 26.9); one and more warps at 16: no gain.
+constexpr int JL_WARPS = 4;
+constexpr uint32_t JL_MAX_LD = 64, JL_CLAIM = 8;
+constexpr uint32_t JL_BUF = 256;   // offers a warp collects before it appends them
+constexpr size_t JL_SMEM_BUDGET = 48 * 1024;
+__host__ __device__ constexpr int jl_partners(int ld) { return ld == 16 ? 2 : 1; }   // per lane, as many as the registers hold
+__host__ __device__ constexpr int jl_blocks(int ld) { return ld <= 32 ? 5 : 4; }
+__host__ __device__ constexpr uint32_t jl_new(uint32_t ld) { return ld <= 48 ? 32 : 16; }   // new entries staged at a time
+// Shared memory per warp: the offer buffer, the new entries' rows, per new entry
+// {norm term, radius, id}, per list entry its id.
+__host__ __device__ constexpr uint32_t jl_warp_bytes(uint32_t cap, uint32_t ld) {
+    return JL_BUF * 8 + jl_new(ld) * (ld * 4 + 16) + (cap + 3) / 4 * 16;
+}
+
+// The canonical raw sum (group4_raw) of a row in shared memory and one in registers.
+template <int LD, bool L2>
+__device__ __forceinline__ float jl_raw(const float *x, const float (&y)[LD], int tail) {
+    constexpr int LAST = LD - 16;
+    auto prod = [](float a, float b) {
+        if (L2) { a = __fsub_rn(a, b); b = a; }
+        return __fmul_rn(a, b);
+    };
+    float r = 0.f;
+    if (LAST > 0 || tail == 0) {
+        float acc[16];
+#pragma unroll
+        for (int c = 0; c < LD; c += 16) {
+            if (c == LAST && tail) break;
+#pragma unroll
+            for (int k = 0; k < 16; k += 4) {
+                const float4 v = ld4(x + c + k);
+                const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float p = prod(e[i], y[c + k + i]);
+                    acc[k + i] = c ? __fadd_rn(acc[k + i], p) : p;
+                }
+            }
+        }
+        float q[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            q[i] = __fadd_rn(__fadd_rn(acc[i], acc[4 + i]), __fadd_rn(acc[8 + i], acc[12 + i]));
+        // the sums start from +0 there: only an all -0 sum differs, and this makes it +0
+        r = __fadd_rn(__fadd_rn(__fadd_rn(q[0], q[1]), __fadd_rn(q[2], q[3])), 0.f);
+    }
+    if (tail) {
+        auto fma1 = [&](int i) {
+            float a = x[LAST + i], b = y[LAST + i];
+            if (L2) { a = __fsub_rn(a, b); b = a; }
+            r = __fmaf_rn(a, b, r);
+        };
+        if (tail >= 8) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) r = __fadd_rn(r, prod(x[LAST + i], y[LAST + i]));
+#pragma unroll
+            for (int i = 8; i < 15; ++i) if (i < tail) fma1(i);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 7; ++i) if (i < tail) fma1(i);
+        }
+    }
+    return r;
+}
+
+template <int LD, bool L2>
+__global__ void __launch_bounds__(JL_WARPS * 32, jl_blocks(LD)) join_lane_kernel(const __grid_constant__ BuildState s) {
+    constexpr int P = jl_partners(LD);
+    constexpr uint32_t JL_NEW = jl_new(LD);
+    extern __shared__ __align__(16) float jl_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    const uint32_t N = s.D.n;
+    const int tail = (int)s.D.d & 15, metric = s.D.metric;
+    unsigned char *wb = reinterpret_cast<unsigned char *>(jl_smem) +
+                        (size_t)warp * jl_warp_bytes(s.NEWCAP + s.OLDCAP, LD);
+    uint2 *buf = reinterpret_cast<uint2 *>(wb);
+    float *rows = reinterpret_cast<float *>(buf + JL_BUF);
+    float4 *info = reinterpret_cast<float4 *>(rows + (size_t)JL_NEW * LD);
+    uint32_t *uid = reinterpret_cast<uint32_t *>(info + JL_NEW);
+    uint32_t comps = 0;   // per lane
+    unsigned long long all = 0;
+    uint32_t next = 0;
+    if (lane == 0) next = s.node_lo + atomicAdd(s.work, JL_CLAIM);
+    for (;;) {
+        const uint32_t base = __shfl_sync(FULL, next, 0);
+        if (base >= s.node_hi) break;
+        if (lane == 0) next = s.node_lo + atomicAdd(s.work, JL_CLAIM);   // needed when this run is done
+        const bool in = lane < (int)JL_CLAIM && base + lane < s.node_hi;
+        const uint32_t ca = in ? min(s.cnt_new[base + lane], s.NEWCAP) : 0u;
+        const uint32_t cb = in ? min(s.cnt_old[base + lane], s.OLDCAP) : 0u;
+        if (in && !ca) s.found[base + lane] = 0u;   // no new entries: no pairs
+        for (unsigned todo = __ballot_sync(FULL, ca > 0); todo; todo &= todo - 1) {
+            const int at = __ffs(todo) - 1;
+            const uint32_t n = base + at, a = __shfl_sync(FULL, ca, at), U = a + __shfl_sync(FULL, cb, at);
+            const uint32_t *nw = s.nn_new + (size_t)n * s.NEWCAP, *od = s.nn_old + (size_t)n * s.OLDCAP;
+            for (uint32_t u = lane; u < U; u += 32) {
+                uint32_t id = u < a ? nw[u] : od[u - a];
+                if (id >= N) { raise_error(s.err, ERR_BAD_ID); id = NO_ID; }
+                uid[u] = id;
+            }
+            __syncwarp();
+            bool uu = false;
+            uint32_t bcnt = 0;
+            for (uint32_t ib = 0; ib < a; ib += JL_NEW) {
+                const uint32_t na = min(a - ib, JL_NEW);
+                for (uint32_t k = lane; k < na * (LD / 4); k += 32) {
+                    const uint32_t r = k / (LD / 4), c = 4 * (k % (LD / 4)), id = uid[ib + r] == NO_ID ? 0u : uid[ib + r];
+                    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(rows + r * LD + c);
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(s.D.X + (size_t)id * LD + c) : "memory");
+                }
+                for (uint32_t u = lane; u < na; u += 32) {
+                    const uint32_t id = uid[ib + u];
+                    // the radii as the join starts (they change only in the merge after it)
+                    const float nr = (id != NO_ID && !L2) ? s.D.norms[id] : 0.f;
+                    const float rd = id != NO_ID ? *reinterpret_cast<volatile float *>(s.radius + id) : 0.f;
+                    info[u] = make_float4(nr, rd, __uint_as_float(id), 0.f);
+                }
+                for (uint32_t jb = ib + 1; jb < U; jb += 32 * P) {
+                    float y[P][LD], nj[P], radj[P];
+                    uint32_t jid[P], lim[P];   // new entries i < lim are this partner's pairs
+#pragma unroll
+                    for (int p = 0; p < P; ++p) {
+                        const uint32_t u = jb + 32 * p + lane;
+                        jid[p] = u < U ? uid[u] : NO_ID;
+                        const bool ok = jid[p] != NO_ID;
+                        lim[p] = ok ? u : 0u;
+                        const size_t id = ok ? jid[p] : 0u;
+                        nj[p] = L2 ? 0.f : s.D.norms[id];
+                        radj[p] = *reinterpret_cast<volatile float *>(s.radius + id);
+#pragma unroll
+                        for (int k = 0; k < LD; k += 4) {
+                            const float4 v = ld4(s.D.X + id * LD + k);
+                            y[p][k] = v.x; y[p][k + 1] = v.y; y[p][k + 2] = v.z; y[p][k + 3] = v.w;
+                        }
+                    }
+                    if (jb == ib + 1) {   // the new entries' rows and terms
+                        asm volatile("cp.async.wait_all;" ::: "memory");
+                        __syncwarp();
+                    }
+                    const uint32_t ie = min(ib + na, jb + 32 * P - 1);
+#pragma unroll 1
+                    for (uint32_t i = ib; i < ie; ++i) {
+                        const float4 f = info[i - ib];
+                        const uint32_t idi = __float_as_uint(f.z);
+#pragma unroll
+                        for (int p = 0; p < P; ++p) {
+                            if (p && jb + 32 * p >= U) break;   // warp-uniform
+                            const float raw = jl_raw<LD, L2>(rows + (i - ib) * LD, y[p], tail);
+                            const float dd = L2 ? raw : finish_metric(raw, f.x, nj[p], metric);
+                            const uint32_t u = jb + 32 * p + lane;
+                            const bool is_nn = u < a;
+                            // i < j by id excludes equal ids among the new entries (kgraph.cpp:742-743)
+                            const bool ok = i < lim[p] && idi != NO_ID && !(is_nn && jid[p] == idi);
+                            comps += ok;
+                            // the unlocked radius test of both directions (kgraph.cpp:725)
+                            const bool ti = ok && !(dd > f.y), tj = ok && !(dd > radj[p]);
+                            const unsigned mi = __ballot_sync(FULL, ti), mj = __ballot_sync(FULL, tj);
+                            if (!(mi | mj)) continue;
+                            const uint32_t ix = (!is_nn || idi < jid[p]) ? JT_UU : 0u;   // the new entry is the pair's x
+                            if (ti) buf[bcnt + __popc(mi & below)] = make_uint2(i | u << 15 | ix, __float_as_uint(dd));
+                            bcnt += __popc(mi);
+                            if (tj) buf[bcnt + __popc(mj & below)] = make_uint2(u | i << 15 | (ix ^ JT_UU), __float_as_uint(dd));
+                            bcnt += __popc(mj);
+                            if (bcnt > JL_BUF - 64) {
+                                __syncwarp();
+                                uu |= jt_flush(s, buf, uid, n, bcnt, lane);
+                                bcnt = 0;
+                            }
+                        }
+                    }
+                }
+                asm volatile("cp.async.wait_all;" ::: "memory");   // (a list of one: nothing waited for it)
+                __syncwarp();   // the staged rows are free again
+            }
+            if (bcnt) {
+                __syncwarp();
+                uu |= jt_flush(s, buf, uid, n, bcnt, lane);
+            }
+            if (lane == 0) s.found[n] = uu;
+            all += comps;
+            comps = 0;
+            __syncwarp();   // the lists are free again
+        }
+    }
+    for (int o = 16; o; o >>= 1) all += __shfl_xor_sync(FULL, all, o);
+    if (lane == 0 && all) atomicAdd(s.n_comps, all);
+}
+
+// The kernel for rows of ld columns, or none.
+const void *join_lane_variant(uint32_t ld, int metric) {
+    const bool l2 = metric == METRIC_L2SQR;
+    if (ld == 16) return l2 ? (const void *)join_lane_kernel<16, true> : (const void *)join_lane_kernel<16, false>;
+    if (ld == 32) return l2 ? (const void *)join_lane_kernel<32, true> : (const void *)join_lane_kernel<32, false>;
+    if (ld == 48) return l2 ? (const void *)join_lane_kernel<48, true> : (const void *)join_lane_kernel<48, false>;
+    if (ld == 64) return l2 ? (const void *)join_lane_kernel<64, true> : (const void *)join_lane_kernel<64, false>;
+    return nullptr;
+}
+
 // ------------------------------------------------------------------ deferred inserts
 // Offers of one join grouped by target: off_grp[off_pos[x] ..) holds x's.
 __global__ void offer_scatter_kernel(BuildState s) {
@@ -1406,6 +1618,11 @@ extern "C" int kg_build(kg_ctx *ctx, const kg_index_params *params, kg_index_inf
                 return cuda_fail(ctx, e, "join");
         }
     }
+    // narrow rows: a lane per pair, where a CTA's lists fit (measured at join_lane_kernel)
+    const void *jl_fn = s.jt_rows && s.D.ld <= JL_MAX_LD ? join_lane_variant(s.D.ld, s.D.metric) : nullptr;
+    const size_t jl_smem = (size_t)JL_WARPS * jl_warp_bytes(s.NEWCAP + s.OLDCAP, s.D.ld);
+    if (jl_smem > JL_SMEM_BUDGET) jl_fn = nullptr;
+    const int jl_grid = (int)std::min<size_t>(jl_blocks((int)s.D.ld), (228u << 10) / (jl_smem + 1024)) * ctx->num_sms;
     // Deferred inserts of the FP32 join: the offer records (linear and grouped,
     // 16 bytes each) hold up to 1024 offers per node within 30 % of the free
     // device memory and 20 GB; the per-target counts, cursors and offsets.
@@ -1529,7 +1746,11 @@ extern "C" int kg_build(kg_ctx *ctx, const kg_index_params *params, kg_index_inf
             sr.node_hi = (uint32_t)((uint64_t)N * (r + 1) / join_rounds);
             cudaMemsetAsync(s.work, 0, 4, st);
             if (s.off_lin) rec_offers_begin();
-            if (s.jt_rows && s.D.metric == METRIC_L2SQR)
+            if (s.jt_rows && jl_fn) {
+                void *args[] = {&sr};
+                cudaError_t e2 = cudaLaunchKernel(jl_fn, dim3(jl_grid), dim3(JL_WARPS * 32), args, jl_smem, st);
+                if (e2 != cudaSuccess) return e2;
+            } else if (s.jt_rows && s.D.metric == METRIC_L2SQR)
                 join_tile_kernel<true><<<ctx->num_sms * jt_blocks, JT_WARPS * 32, jt_smem, st>>>(sr);
             else if (s.jt_rows)
                 join_tile_kernel<false><<<ctx->num_sms * jt_blocks, JT_WARPS * 32, jt_smem, st>>>(sr);
