@@ -73,7 +73,7 @@ struct JoinQueue {
     uint32_t *work;      // claim counter within a round
     uint32_t *bounds;    // round boundaries (node ids)
 };
-constexpr int JOIN_TC_MAX_CTAS_PER_SM = 3;
+constexpr int JOIN_TC_MAX_CTAS_PER_SM = 6;
 // Fraction of full pools (finite radii) from which an iteration's join runs
 // on the tensor cores.
 constexpr double JOIN_TC_MIN_FULL = 0.5;

@@ -12,18 +12,21 @@
 //      distances -- instead of the raw norms.  The same pass keeps, per row,
 //      h = |x_u - x_n|^2 / 2 and c = (x_u - x_n) . x_n in FP32.
 //   2. tcgen05.mma (kind::f16, BF16 x BF16 -> FP32 in TMEM) forms the Gram
-//      block of U (128-row tiles, M) against the new rows (128-column tiles,
-//      N); the new rows are the first rows of U, so B is read from the same
-//      staged buffer.
+//      block of 32 new rows (N) against themselves and 96 of the entries after
+//      them (M = 128); the new rows are the tile's first 32, so B is read from
+//      the same staged buffer.  A node has 10 to 30 new entries and 20 to 70 in
+//      all: with 128 columns and a second 128-row buffer an SM held three CTAs
+//      of eight warps, half of them without a row; four warps, 32 TMEM columns
+//      and one buffer make that six nodes at a time, each with its next list in
+//      flight.  200k x 96 (K=50 L=100 S=12) whole build 178 -> 153 ms, 100k x
+//      128 97 -> 79, 60k x 64 36 -> 28; E4M3 tiles 200k x 96 331 -> 290.
 //   3. Each epilogue thread owns one U row (one TMEM lane) and derives the
 //      approximate distance of each of its pairs: euclidean h_u + h_j - g,
 //      l2sqr twice that, angular -(g + c_u + c_j + |x_n|^2) / (n_u n_j + eps).
 //      The test is arranged so that a pair costs a dozen multiply-adds
 //      (filter_terms): with a square root and a division per pair this epilogue
 //      was two thirds of the kernel (200k x 96 unit-norm mixture, K=50 L=100
-//      S=12, whole build 386 -> 193 ms; E4M3 tiles 551 -> 345 ms), and the two
-//      warps of a lane quadrant take alternating 16-column pieces, so both work
-//      where a node has at most 32 new entries.
+//      S=12, whole build 386 -> 193 ms; E4M3 tiles 551 -> 345 ms).
 //      A pair whose approximate distance minus a rigorous error margin E is
 //      above BOTH endpoints' radius cannot pass the reference's unlocked
 //      radius test (kgraph.cpp:725, radii only shrink during a join), so it is
@@ -53,13 +56,13 @@
 namespace kgb {
 namespace {
 
-constexpr int TC_THREADS = 256;          // 8 warps: warp w reads TMEM lanes 32*(w%4).., columns 16*(2k + w/4)..
-constexpr uint32_t TC_M = 128;           // U rows per tile = TMEM lanes
-constexpr uint32_t TC_N = 128;           // new columns per tile = TMEM columns
-constexpr uint32_t TC_TMEM_COLS = 128;
+constexpr int TC_THREADS = 128;          // warp w reads TMEM lanes 32 w .. 32 w + 31
+constexpr uint32_t TC_M = 128;           // rows per tile = TMEM lanes
+constexpr uint32_t TC_N = 32;            // new columns per tile = TMEM columns
+constexpr uint32_t TC_REST = TC_M - TC_N;   // partners per tile besides the columns' own rows
+constexpr uint32_t TC_TMEM_COLS = 32;
 constexpr long long TC_WAIT_CYCLES = 2000000000ll;
-constexpr uint32_t TC_CLAIM = 16;               // nodes claimed per CTA at a time
-constexpr uint32_t TC_MIN_SMEM = 58 * 1024;   // at most 3 CTAs (384 TMEM columns) per SM
+constexpr uint32_t TC_CLAIM = 8;         // nodes claimed per CTA at a time
 
 __device__ __forceinline__ bool sampled_node(uint32_t n) { return ((n * 0x9E3779B1u) >> 21) == 0; }
 
@@ -111,7 +114,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 
 struct TcShared {
-    uint8_t *bbuf, *abuf;   // two 128-row tiles (BF16 or E4M3), K-major core-matrix layout
+    uint8_t *buf;           // the 128-row tile (BF16 or E4M3), K-major core-matrix layout
     float *xn;              // x_n, FP32
     float4 *tA;             // per U row {A, s, radius, id (NO_ID for a bad id)} (filter_terms)
     float2 *tC;             // {C, canonical norm term}
@@ -143,13 +146,26 @@ __device__ __forceinline__ void filter_terms(int metric, float h, float c, float
     }
 }
 
-// Rows [u0, u0 + rows) of U into `buf` (all 128 tile rows written; rows past
-// `rows` are zero).  Warp w stages row groups w, w+8: lane l owns row
-// (l & 7) of the group and 16-byte chunks (l >> 3) + 4i, so each quarter-warp
-// store covers one contiguous 128-byte core matrix.
+// The tile's rows: entries [j0, j0 + nb) of U in rows 0 .. nb - 1, entries
+// [us, us + nr) in rows 32 .. 32 + nr - 1.  Groups of 8 rows go to the warps in
+// turn: lane l owns row (l & 7) of the group and 16-byte chunks (l >> 3) + 4i, so
+// each quarter-warp store covers one contiguous 128-byte core matrix.
+struct TileRows {
+    uint32_t j0, nb, us, nr;
+    __device__ __forceinline__ uint32_t groups() const { return (nb + 7) / 8 + (nr + 7) / 8; }
+    // row r = 8 g + k of the staging order: its tile row and entry; false past the end
+    __device__ __forceinline__ bool at(uint32_t g, uint32_t k, uint32_t &row, uint32_t &u) const {
+        const uint32_t gb = (nb + 7) / 8;
+        const bool first = g < gb;
+        const uint32_t r = (first ? g : g - gb) * 8 + k;
+        row = first ? r : TC_N + r;
+        u = (first ? j0 : us) + r;
+        return r < (first ? nb : nr);
+    }
+};
 template <int PREC>
-__device__ void stage_rows(const BuildState &s, const TcShared &sh, uint8_t *buf, uint32_t u0, uint32_t rows,
-                           float qn, float gam, int warp, int lane);
+__device__ void stage_rows(const BuildState &s, const TcShared &sh, const TileRows &tr, float qn, float gam, int warp,
+                           int lane);
 
 // E4M3 rows with a per-row scale: v = x_u - x_n in FP32 (as the BF16 rows),
 // scale = max|v| / 448, q = e4m3_satfinite(v / scale); per row the exact
@@ -157,13 +173,13 @@ __device__ void stage_rows(const BuildState &s, const TcShared &sh, uint8_t *buf
 // Lane l owns row (l & 7) of a group of 8 and 16-byte chunks (16 elements)
 // (l >> 3) + 4i; the row's maximum needs a first pass over its elements.
 template <>
-__device__ void stage_rows<1>(const BuildState &s, const TcShared &sh, uint8_t *buf, uint32_t u0, uint32_t rows,
-                              float qn, float gam, int warp, int lane) {
+__device__ void stage_rows<1>(const BuildState &s, const TcShared &sh, const TileRows &tr, float qn, float gam,
+                              int warp, int lane) {
     const uint32_t Dp = s.D.ld, nk16 = Dp >> 4;
-    for (uint32_t g = warp; g * 8 < rows; g += TC_THREADS / 32) {
-        const uint32_t rl = g * 8 + (lane & 7);
-        const bool valid = rl < rows;
-        const uint32_t id = valid ? __float_as_uint(sh.tA[u0 + rl].w) : NO_ID;
+    for (uint32_t g = warp; g < tr.groups(); g += TC_THREADS / 32) {
+        uint32_t rl, u;
+        const bool valid = tr.at(g, lane & 7, rl, u);
+        const uint32_t id = valid ? __float_as_uint(sh.tA[u].w) : NO_ID;
         const bool ok = id != NO_ID;
         float nrm = 0.f, rd = -FLT_MAX;
         if (ok && lane < 8) {
@@ -209,12 +225,11 @@ __device__ void stage_rows<1>(const BuildState &s, const TcShared &sh, uint8_t *
                 }
                 wv[h] = word;
             }
-            *reinterpret_cast<uint4 *>(buf + tc::kmajor_off8(rl, 16 * k16, Dp)) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+            *reinterpret_cast<uint4 *>(sh.buf + tc::kmajor_off8(rl, 16 * k16, Dp)) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
         }
         err2 += __shfl_xor_sync(FULL, err2, 8);
         err2 += __shfl_xor_sync(FULL, err2, 16);
         if (lane < 8 && valid) {
-            const uint32_t u = u0 + rl;
             filter_terms(s.D.metric, 0.5f * hs, cs, nrm, qn, gam, rd, id, sh.tA[u], sh.tC[u]);
             // relative to ||v|| (hs carries an FP32 rounding: one more relative step of slack)
             const float rel = hs > 0.f ? __double2float_ru(sqrt(err2) / sqrt((double)hs) * (1.0 + 1e-5)) : 0.f;
@@ -225,15 +240,15 @@ __device__ void stage_rows<1>(const BuildState &s, const TcShared &sh, uint8_t *
 }
 
 template <>
-__device__ void stage_rows<0>(const BuildState &s, const TcShared &sh, uint8_t *buf, uint32_t u0, uint32_t rows,
-                              float qn, float gam, int warp, int lane) {
+__device__ void stage_rows<0>(const BuildState &s, const TcShared &sh, const TileRows &tr, float qn, float gam,
+                              int warp, int lane) {
     const uint32_t Dp = s.D.ld, nk8 = Dp >> 3;
-    // Rows past `rows` are left as they are: the MMA reads them, but their
+    // Rows past nb and nr are left as they are: the MMA reads them, but their
     // products land only in masked rows / columns of the accumulator.
-    for (uint32_t g = warp; g * 8 < rows; g += TC_THREADS / 32) {
-        const uint32_t rl = g * 8 + (lane & 7);
-        const bool valid = rl < rows;
-        const uint32_t id = valid ? __float_as_uint(sh.tA[u0 + rl].w) : NO_ID;
+    for (uint32_t g = warp; g < tr.groups(); g += TC_THREADS / 32) {
+        uint32_t rl, u;
+        const bool valid = tr.at(g, lane & 7, rl, u);
+        const uint32_t id = valid ? __float_as_uint(sh.tA[u].w) : NO_ID;
         const bool ok = id != NO_ID;
         float nrm = 0.f, rd = -FLT_MAX;
         if (ok && lane < 8) {   // issued ahead of the row loads
@@ -262,14 +277,13 @@ __device__ void stage_rows<0>(const BuildState &s, const TcShared &sh, uint8_t *
             uint4 pk;
             pk.x = pack_bf16(e[0], e[1]); pk.y = pack_bf16(e[2], e[3]);
             pk.z = pack_bf16(e[4], e[5]); pk.w = pack_bf16(e[6], e[7]);
-            *reinterpret_cast<uint4 *>(buf + tc::kmajor_off(rl, 8 * k8, Dp)) = pk;
+            *reinterpret_cast<uint4 *>(sh.buf + tc::kmajor_off(rl, 8 * k8, Dp)) = pk;
         }
         hs += __shfl_xor_sync(FULL, hs, 8);
         hs += __shfl_xor_sync(FULL, hs, 16);
         cs += __shfl_xor_sync(FULL, cs, 8);
         cs += __shfl_xor_sync(FULL, cs, 16);
         if (lane < 8 && valid) {
-            const uint32_t u = u0 + rl;
             filter_terms(s.D.metric, 0.5f * hs, cs, nrm, qn, gam, rd, id, sh.tA[u], sh.tC[u]);
         }
     }
@@ -277,22 +291,19 @@ __device__ void stage_rows<0>(const BuildState &s, const TcShared &sh, uint8_t *
 }
 
 template <int PREC>
-__global__ void __launch_bounds__(TC_THREADS, 3) join_tc_kernel(BuildState s, uint32_t Umax, JoinQueue jq,
+__global__ void __launch_bounds__(TC_THREADS, JOIN_TC_MAX_CTAS_PER_SM) join_tc_kernel(BuildState s, uint32_t Umax, JoinQueue jq,
                                                                   uint32_t round) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t mbar;
-    __shared__ uint32_t tmem_base, s_base, s_cnt;
+    __shared__ uint32_t tmem_base, s_cnt;
     __shared__ uint32_t s_list[TC_CLAIM], s_la[TC_CLAIM], s_lb[TC_CLAIM];
-    __shared__ uint32_t s_wcnt[TC_THREADS / 32];
-    __shared__ unsigned long long s_wbase[TC_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t Dp = s.D.ld, N = s.D.n;
     const uint32_t n_begin = jq.bounds[round], n_end = jq.bounds[round + 1];
     const uint32_t tile_bytes = TC_M * Dp * (PREC ? 1 : 2);
     TcShared sh;
-    sh.bbuf = smem;
-    sh.abuf = smem + tile_bytes;
-    sh.xn = reinterpret_cast<float *>(smem + 2 * tile_bytes);
+    sh.buf = smem;
+    sh.xn = reinterpret_cast<float *>(smem + tile_bytes);
     sh.tA = reinterpret_cast<float4 *>(sh.xn + Dp);   // 16-byte aligned: Dp is a multiple of 16
     sh.tC = reinterpret_cast<float2 *>(sh.tA + Umax + TC_PAD);
     sh.tF = sh.tC + Umax + TC_PAD;
@@ -303,7 +314,6 @@ __global__ void __launch_bounds__(TC_THREADS, 3) join_tc_kernel(BuildState s, ui
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tmem_base;
-    const int q = warp & 3, half = warp >> 2;
     const float et = 0.00390625f + 7.63e-6f + (float)(s.D.d + 4) * 1.1921e-7f;   // 2^-8 + 2^-17 + (D+4) 2^-23
     // E4M3 tiles: the products' FP32 accumulation, allowed 2^-20 per add, and the two scale multiplies
     const float g8 = (float)(s.D.d + 4) * 9.5367e-7f + 8.f * 5.9605e-8f;
@@ -313,14 +323,12 @@ __global__ void __launch_bounds__(TC_THREADS, 3) join_tc_kernel(BuildState s, ui
     bool aborted = false;
     unsigned long long comps = 0, passed = 0;
 
+    uint32_t next = 0;
+    if (tid == 0) next = n_begin + atomicAdd(jq.work, TC_CLAIM);
     for (;;) {
         // claim TC_CLAIM nodes of this round's range; keep those with new entries
-        if (tid == 0) s_base = n_begin + atomicAdd(jq.work, TC_CLAIM);
-        __syncthreads();
-        const uint32_t base = s_base;
-        if (base >= n_end) break;
         if (warp == 0) {
-            const uint32_t nn = base + lane;
+            const uint32_t base = __shfl_sync(FULL, next, 0), nn = base + lane;
             bool act = false;
             uint32_t ca = 0, cb = 0;
             if (lane < (int)TC_CLAIM && nn < n_end) {
@@ -332,92 +340,106 @@ __global__ void __launch_bounds__(TC_THREADS, 3) join_tc_kernel(BuildState s, ui
             const unsigned am = __ballot_sync(FULL, act);
             if (act) {
                 const int slot = __popc(am & ((1u << lane) - 1u));
+                if (ca > s.NEWCAP || cb > s.OLDCAP) raise_error(s.err, ERR_CAPACITY);
                 s_list[slot] = nn;
-                s_la[slot] = ca;
-                s_lb[slot] = cb;
+                s_la[slot] = min(ca, s.NEWCAP);
+                s_lb[slot] = min(cb, s.OLDCAP);
             }
-            if (lane == 0) s_cnt = __popc(am);
+            if (lane == 0) {
+                s_cnt = base < n_end ? __popc(am) : NO_ID;
+                if (base < n_end) next = n_begin + atomicAdd(jq.work, TC_CLAIM);   // needed when this run is done
+            }
         }
         __syncthreads();
         const uint32_t cnt = s_cnt;
+        if (cnt == NO_ID) break;
+        // a node's list and row are read one node ahead: the first two entries a
+        // thread takes of it, and this thread's column of x_n
+        uint32_t pid[2] = {0u, 0u};
+        float px = 0.f;
+        auto entry = [&](uint32_t n, uint32_t a, uint32_t u) {
+            return u < a ? s.nn_new[(size_t)n * s.NEWCAP + u] : s.nn_old[(size_t)n * s.OLDCAP + u - a];
+        };
+        auto fetch = [&](uint32_t li) {
+            if (li >= cnt) return;
+            const uint32_t n = s_list[li], a = s_la[li], U = a + s_lb[li];
+#pragma unroll
+            for (uint32_t k = 0; k < 2; ++k)
+                if (tid + k * TC_THREADS < U) pid[k] = entry(n, a, tid + k * TC_THREADS);
+            if (tid < Dp) px = s.D.X[(size_t)n * Dp + tid];
+        };
+        fetch(0);
         for (uint32_t li = 0; li < cnt && !aborted; ++li) {
-        const uint32_t n = s_list[li];
-        uint32_t a = s_la[li], b = s_lb[li];
-        if (a > s.NEWCAP || b > s.OLDCAP) {
-            if (tid == 0) raise_error(s.err, ERR_CAPACITY);
-            a = min(a, s.NEWCAP);
-            b = min(b, s.OLDCAP);
-        }
+        const uint32_t n = s_list[li], a = s_la[li], b = s_lb[li];
         const uint32_t U = a + b;
-        const uint32_t *nw = s.nn_new + (size_t)n * s.NEWCAP, *od = s.nn_old + (size_t)n * s.OLDCAP;
-        for (uint32_t u = tid; u < U; u += TC_THREADS) {
-            uint32_t id = u < a ? nw[u] : od[u - a];
+        auto put = [&](uint32_t u, uint32_t id) {
             if (id >= N) { raise_error(s.err, ERR_BAD_ID); id = NO_ID; }
             sh.tA[u].w = __uint_as_float(id);
-        }
-        const float *xrow = s.D.X + (size_t)n * Dp;
-        for (uint32_t k = tid; k < Dp; k += TC_THREADS) sh.xn[k] = xrow[k];
+        };
+#pragma unroll
+        for (uint32_t k = 0; k < 2; ++k)
+            if (tid + k * TC_THREADS < U) put(tid + k * TC_THREADS, pid[k]);
+        for (uint32_t u = tid + 2 * TC_THREADS; u < U; u += TC_THREADS) put(u, entry(n, a, u));
+        if (tid < Dp) sh.xn[tid] = px;
+        for (uint32_t k = tid + TC_THREADS; k < Dp; k += TC_THREADS) sh.xn[k] = s.D.X[(size_t)n * Dp + k];
         __syncthreads();
+        fetch(li + 1);
         float qn = 0.f;   // |x_n|^2, in every warp
         for (uint32_t k = lane; k < Dp; k += 32) qn += sh.xn[k] * sh.xn[k];
         for (int o = 16; o; o >>= 1) qn += __shfl_xor_sync(FULL, qn, o);
         const bool samp = sampled_node(n);
         for (uint32_t j0 = 0; j0 < a && !aborted; j0 += TC_N) {
-            const uint32_t j1 = min(a, j0 + TC_N);
-            stage_rows<PREC>(s, sh, sh.bbuf, j0, min(U, j0 + TC_M) - j0, qn, gam, warp, lane);
-            for (uint32_t u0 = 0; u0 < U; u0 += TC_M) {
-                const uint32_t u1 = min(U, u0 + TC_M);
-                if (!(u1 > max(u0, a) || (u0 < a && u0 + 1 < j1))) continue;   // no pair needed in this tile
-                const bool same = u0 == j0;
-                if (!same) stage_rows<PREC>(s, sh, sh.abuf, u0, u1 - u0, qn, gam, warp, lane);
+            const uint32_t nb = min(TC_N, a - j0);   // new columns [j0, j0 + nb), also the tile's rows 0 .. nb - 1
+            bool first = true;
+            // their partners: the block itself, then the entries after it, TC_REST at a time
+            for (uint32_t us = j0 + nb; first || us < U; us += TC_REST, first = false) {
+                const uint32_t nr = us < U ? min(TC_REST, U - us) : 0u;
+                stage_rows<PREC>(s, sh, TileRows{j0, first ? nb : 0u, us, nr}, qn, gam, warp, lane);
                 tc::fence_before_sync();
                 __syncthreads();
-                if (tid == 0) {
+                if (warp == 0 && tc::elect_one()) {
                     tc::fence_after_sync();
-                    const uint32_t aa = tc::smem_addr(same ? sh.bbuf : sh.abuf), ba = tc::smem_addr(sh.bbuf);
+                    const uint32_t aa = tc::smem_addr(sh.buf);
                     if constexpr (PREC == 1) {   // K = 32 bytes per step, rows of Dp bytes
                         const uint32_t idesc = tc::idesc_e4m3_f32(TC_M, TC_N);
-                        for (uint32_t kk = 0; kk < Dp / 32; ++kk)
-                            tc::mma_e4m3(tmem, tc::smem_desc(aa + kk * 256, 128, Dp * 8),
-                                         tc::smem_desc(ba + kk * 256, 128, Dp * 8), idesc, kk > 0);
+                        for (uint32_t kk = 0; kk < Dp / 32; ++kk) {
+                            const uint64_t de = tc::smem_desc(aa + kk * 256, 128, Dp * 8);
+                            tc::mma_e4m3(tmem, de, de, idesc, kk > 0);
+                        }
                     } else {
                         const uint32_t idesc = tc::idesc_bf16_f32(TC_M, TC_N);
-                        for (uint32_t kk = 0; kk < Dp / 16; ++kk)
-                            tc::mma_bf16(tmem, tc::smem_desc(aa + kk * 256, 128, Dp * 16),
-                                         tc::smem_desc(ba + kk * 256, 128, Dp * 16), idesc, kk > 0);
+                        for (uint32_t kk = 0; kk < Dp / 16; ++kk) {
+                            const uint64_t de = tc::smem_desc(aa + kk * 256, 128, Dp * 16);
+                            tc::mma_bf16(tmem, de, de, idesc, kk > 0);
+                        }
                     }
                     tc::mma_commit(&mbar);
                 }
-                const bool ok = tc::mbar_wait(&mbar, phase, TC_WAIT_CYCLES);
-                if (__syncthreads_or(!ok)) {
-                    if (tid == 0) raise_error(s.err, ERR_TC_TIMEOUT);
-                    aborted = true;
-                    break;
-                }
-                phase ^= 1;
+                const bool ok = __all_sync(FULL, tc::mbar_wait(&mbar, phase, TC_WAIT_CYCLES));
                 tc::fence_after_sync();
 
-                // ---- epilogue: this thread's U row against the columns 16 (2 k + half) .. + 15
-                const uint32_t u = u0 + 32 * q + lane;
-                const float4 ua = u < u1 ? sh.tA[u] : make_float4(0.f, 0.f, 0.f, __uint_as_float(NO_ID));
+                // ---- epilogue: this thread's row against the columns
+                const uint32_t u = warp == 0 ? j0 + lane : us + 32 * (warp - 1) + lane;
+                const bool in = warp == 0 ? first && (uint32_t)lane < nb : u < us + nr;
+                const float4 ua = in ? sh.tA[u] : make_float4(0.f, 0.f, 0.f, __uint_as_float(NO_ID));
                 const bool uval = __float_as_uint(ua.w) != NO_ID;
                 const uint32_t idu = uval ? __float_as_uint(ua.w) : 0u;
                 const bool unew = u < a;
                 const float2 uc = uval ? sh.tC[u] : make_float2(0.f, 0.f);
                 const float2 uf = (PREC == 1 && uval) ? sh.tF[u] : make_float2(1.f, 1.f);
                 const float k2 = 2.f * et * ua.y;
-                const bool wnew = u0 + 32 * q < a;   // the warp holds new rows
-                unsigned pmask[4] = {0u, 0u, 0u, 0u};
+                const bool work = ok && __any_sync(FULL, in);
+                unsigned pmask[2] = {0u, 0u};
 #pragma unroll
-                for (int part = 0; part < 4; ++part) {
-                    const uint32_t cb = 32 * part + 16 * half;
-                    if (j0 + cb >= j1) break;   // warp-uniform
+                for (int part = 0; part < 2; ++part) {
+                    const uint32_t cb = 16 * part;
+                    if (!work || cb >= nb) break;   // warp-uniform
                     float v[16];
-                    tc::tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + cb, v);
-                    // the pairs of this row: columns in range, after the row among the new ones
-                    const uint32_t cols = min(16u, j1 - j0 - cb);
+                    tc::tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + cb, v);
+                    // the pairs of this row: every column, in the block's own rows those after the row
+                    const uint32_t cols = min(16u, nb - cb);
                     unsigned need = uval ? (1u << cols) - 1u : 0u;
-                    if (unew && u >= j0 + cb) need &= u - j0 - cb >= 15 ? 0u : ~0u << (u - j0 - cb + 1);
+                    if (warp == 0 && (uint32_t)lane >= cb) need &= lane - cb >= 15 ? 0u : ~0u << (lane - cb + 1);
                     unsigned pm = 0;
 #pragma unroll
                     for (int c = 0; c < 16; ++c) {
@@ -440,7 +462,7 @@ __global__ void __launch_bounds__(TC_THREADS, 3) join_tc_kernel(BuildState s, ui
                         }
                         if (!skip) pm |= 1u << c;
                         const uint32_t idj = __float_as_uint(ja.w);
-                        if (idj == NO_ID || (wnew && unew && idj == idu)) need &= ~(1u << c);
+                        if (idj == NO_ID || (unew && idj == idu)) need &= ~(1u << c);
                     }
                     pm &= need;
                     comps += __popc(need);
@@ -503,28 +525,21 @@ __global__ void __launch_bounds__(TC_THREADS, 3) join_tc_kernel(BuildState s, ui
                         }
                     }
                 }
-                // append the survivors: one queue atomic per tile
-                const uint32_t mine = __popc(pmask[0]) + __popc(pmask[1]) + __popc(pmask[2]) + __popc(pmask[3]);
+                // append the survivors: one queue atomic per warp
+                const uint32_t mine = __popc(pmask[0]) + __popc(pmask[1]);
                 uint32_t incl = mine;
                 for (int o = 1; o < 32; o <<= 1) {
                     const uint32_t t = __shfl_up_sync(FULL, incl, o);
                     if (lane >= o) incl += t;
                 }
-                if (lane == 31) s_wcnt[warp] = incl;
-                __syncthreads();
-                if (tid == 0) {
-                    unsigned long long tot = 0;
-                    for (int w = 0; w < TC_THREADS / 32; ++w) { s_wbase[w] = tot; tot += s_wcnt[w]; }
-                    const unsigned long long b0 = tot ? atomicAdd(jq.tail, tot) : 0ull;
-                    for (int w = 0; w < TC_THREADS / 32; ++w) s_wbase[w] += b0;
-                }
-                __syncthreads();
-                unsigned long long pos = s_wbase[warp] + incl - mine;
+                unsigned long long pos = 0;
+                if (lane == 31 && incl) pos = atomicAdd(jq.tail, (unsigned long long)incl);
+                pos = __shfl_sync(FULL, pos, 31) + incl - mine;
                 passed += mine;
 #pragma unroll
-                for (int part = 0; part < 4; ++part) {
+                for (int part = 0; part < 2; ++part) {
                     unsigned pm = pmask[part];
-                    const uint32_t cb = 32 * part + 16 * half;
+                    const uint32_t cb = 16 * part;
                     while (pm) {
                         const int c = __ffs(pm) - 1;
                         pm &= pm - 1;
@@ -536,12 +551,17 @@ __global__ void __launch_bounds__(TC_THREADS, 3) join_tc_kernel(BuildState s, ui
                     }
                 }
                 tc::fence_before_sync();
-                __syncthreads();   // TMEM and the A tile are free again
+                if (__syncthreads_or(!ok)) {   // TMEM and the tile are free again
+                    if (tid == 0) raise_error(s.err, ERR_TC_TIMEOUT);
+                    aborted = true;
+                    break;
+                }
+                phase ^= 1;
             }
         }
-        __syncthreads();   // this node's shared arrays are free again
         }
         if (aborted) break;
+        __syncthreads();   // the claimed list is free again
     }
 
     if (aborted) tc::mbar_wait(&mbar, phase, TC_WAIT_CYCLES);   // the MMA still in flight, bounded
@@ -622,15 +642,17 @@ __global__ void join_bounds_kernel(const uint64_t *pre, uint32_t N, uint64_t sla
     }
 }
 
+size_t join_tc_tile(const BuildState &s, int prec) { return (size_t)TC_M * s.D.ld * (prec ? 1 : 2); }
 size_t join_tc_smem(const BuildState &s, int prec) {
     const size_t Umax = (size_t)s.NEWCAP + s.OLDCAP;
-    return 2 * (size_t)TC_M * s.D.ld * (prec ? 1 : 2) + (size_t)s.D.ld * 4 + (Umax + TC_PAD) * (prec ? 32 : 24);
+    return join_tc_tile(s, prec) + (size_t)s.D.ld * 4 + (Umax + TC_PAD) * (prec ? 32 : 24);
 }
 
 }  // namespace
 
 bool join_tc_supported(const BuildState &s, int prec) {
-    return s.D.ld % (prec ? 32 : 16) == 0 && join_tc_smem(s, prec) <= 224 * 1024;   // with the static part, within a CTA's 227 KB
+    // two CTAs an SM at least; wider rows take the CUDA-core join
+    return s.D.ld % (prec ? 32 : 16) == 0 && join_tc_smem(s, prec) + join_tc_tile(s, prec) <= 224 * 1024;
 }
 
 uint64_t join_tc_node_max(const BuildState &s) {
@@ -651,8 +673,7 @@ cudaError_t join_tc_bounds(cudaStream_t st, const uint64_t *pre, uint32_t N, uin
 cudaError_t launch_join_tc(int num_sms, int grid_insert, cudaStream_t st, const BuildState &s, JoinQueue jq,
                            uint32_t round, int prec) {
     auto kern = prec ? join_tc_kernel<1> : join_tc_kernel<0>;
-    size_t smem = join_tc_smem(s, prec);
-    if (smem < TC_MIN_SMEM) smem = TC_MIN_SMEM;
+    const size_t smem = join_tc_smem(s, prec);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
