@@ -71,9 +71,15 @@ struct JoinQueue {
     uint32_t *x, *y, *n;
     unsigned long long *tail;
     uint32_t *work;      // claim counter within a round
+    uint32_t *stail;     // sampled pairs of the round (recorded while below JOIN_TC_SAMPLES)
+    uint4 *sample;       // {node, rows, Gram entry} of a sampled pair, and its product error
+    float *setp;
     uint32_t *bounds;    // round boundaries (node ids)
 };
 constexpr int JOIN_TC_MAX_CTAS_PER_SM = 6;
+// Sampled pairs recorded in a round: eight times what a full queue's nodes give
+// on average (1 in 2048 is sampled); beyond it they are evaluated where found.
+constexpr uint32_t JOIN_TC_SAMPLES = 1u << 18;
 // Fraction of full pools (finite radii) from which an iteration's join runs
 // on the tensor cores.
 constexpr double JOIN_TC_MIN_FULL = 0.5;

@@ -108,6 +108,61 @@ __device__ double warp_dist64(const DataView &D, uint32_t i, uint32_t j, int lan
     return D.metric == METRIC_L2SQR ? s : 0.5 * s;
 }
 
+// What a warp's sampled pairs add to the join's statistics.
+struct SampleTally {
+    unsigned long long sampled, violations, rel_count;
+    double sum_abs, sum_ratio, sum_rel;
+    uint32_t max_abs, max_ratio, max_rel;   // bits of non-negative floats
+    __device__ void add(JoinTcStats *t) const {
+        atomicAdd(&t->sampled, sampled);
+        atomicAdd(&t->sum_abs, sum_abs);
+        atomicAdd(&t->sum_ratio, sum_ratio);
+        atomicMax(&t->max_abs_bits, max_abs);
+        atomicMax(&t->max_ratio_bits, max_ratio);
+        if (rel_count) {
+            atomicAdd(&t->rel_count, rel_count);
+            atomicAdd(&t->sum_rel, sum_rel);
+            atomicMax(&t->max_rel_bits, max_rel);
+        }
+        if (violations) atomicAdd(&t->violations, violations);
+    }
+};
+
+// Whole warp: the error of the approximate distance of rows ia and ib of node
+// n's lists (Gram entry g, product error etp) against FP64.
+__device__ __noinline__ void sample_pair(const BuildState &s, uint32_t n, uint32_t ia, uint32_t ib, float g, float etp,
+                                         int lane, SampleTally &t) {
+    const uint32_t Dp = s.D.ld;
+    const float gam = (float)(s.D.d + 4) * 5.9605e-8f;
+    const float *xn = s.D.X + (size_t)n * Dp;
+    float qn = 0.f, hc[4] = {0.f, 0.f, 0.f, 0.f};   // |x_n|^2; h and c of both rows (filter_terms)
+    for (uint32_t k = lane; k < Dp; k += 32) {
+        const float x = xn[k], ea = s.D.X[(size_t)ia * Dp + k] - x, eb = s.D.X[(size_t)ib * Dp + k] - x;
+        qn += x * x;
+        hc[0] += ea * ea; hc[1] += eb * eb; hc[2] += ea * x; hc[3] += eb * x;
+    }
+    for (int o = 16; o; o >>= 1) {
+        qn += __shfl_xor_sync(FULL, qn, o);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) hc[k] += __shfl_xor_sync(FULL, hc[k], o);
+    }
+    const Approx ap = approx_dist(s.D.metric, g, 0.5f * hc[0], 0.5f * hc[1], hc[2], hc[3], s.D.norms[ia], s.D.norms[ib],
+                                  qn, etp, gam);
+    const double d64 = warp_dist64(s.D, ia, ib, lane), err = fabs((double)ap.d - d64), ratio = err / (double)ap.e;
+    ++t.sampled;
+    t.sum_abs += err;
+    t.sum_ratio += ratio;
+    t.max_abs = max(t.max_abs, __float_as_uint((float)err));
+    t.max_ratio = max(t.max_ratio, __float_as_uint((float)ratio));
+    if (d64 != 0.0) {
+        const double rel = err / fabs(d64);
+        ++t.rel_count;
+        t.sum_rel += rel;
+        t.max_rel = max(t.max_rel, __float_as_uint((float)rel));
+    }
+    if (err > (double)ap.e) ++t.violations;
+}
+
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t *>(&v);
@@ -291,8 +346,8 @@ __device__ void stage_rows<0>(const BuildState &s, const TcShared &sh, const Til
 }
 
 template <int PREC>
-__global__ void __launch_bounds__(TC_THREADS, JOIN_TC_MAX_CTAS_PER_SM) join_tc_kernel(BuildState s, uint32_t Umax, JoinQueue jq,
-                                                                  uint32_t round) {
+__global__ void __launch_bounds__(TC_THREADS, JOIN_TC_MAX_CTAS_PER_SM)
+    join_tc_kernel(const __grid_constant__ BuildState s, uint32_t Umax, JoinQueue jq, uint32_t round) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_base, s_cnt;
@@ -467,61 +522,38 @@ __global__ void __launch_bounds__(TC_THREADS, JOIN_TC_MAX_CTAS_PER_SM) join_tc_k
                     pm &= need;
                     comps += __popc(need);
                     pmask[part] = pm;
-                    if (samp) {   // FP64 tile error on this node's pairs, one pair at a time per warp
-                        unsigned nm = need;
-                        for (;;) {
-                            const unsigned any = __ballot_sync(FULL, nm != 0);
-                            if (!any) break;
-                            const int src = __ffs(any) - 1;
-                            uint32_t ia = 0, ib = 0;
-                            float g = 0.f, etp = et;
-                            if (lane == src) {
-                                const int c = __ffs(nm) - 1;
-                                nm &= nm - 1;
-                                const uint32_t j = j0 + cb + c;
+                    if (samp) {   // this node's pairs to the FP64 check
+                        const uint32_t have = __popc(need);
+                        uint32_t end = have;
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const uint32_t t = __shfl_up_sync(FULL, end, o);
+                            if (lane >= o) end += t;
+                        }
+                        uint32_t at = 0;
+                        if (lane == 31 && end) at = atomicAdd(jq.stail, end);
+                        at = __shfl_sync(FULL, at, 31) + end - have;
 #pragma unroll
-                                for (int k = 0; k < 16; ++k) if (k == c) g = v[k];
-                                if constexpr (PREC == 1) {
-                                    g = g * uf.x * sh.tF[j].x;
-                                    etp = uf.y * sh.tF[j].y * (1.f + g8) - 1.f;
-                                }
-                                ia = idu;
-                                ib = __float_as_uint(sh.tA[j].w);
+                        for (int c = 0; c < 16; ++c) {
+                            const bool mine = (need >> c) & 1u;
+                            if (!__any_sync(FULL, mine)) continue;
+                            const uint32_t j = j0 + cb + c;
+                            float g = v[c], etp = et;
+                            if constexpr (PREC == 1) {
+                                g = g * uf.x * sh.tF[j].x;
+                                etp = uf.y * sh.tF[j].y * (1.f + g8) - 1.f;
                             }
-                            ia = __shfl_sync(FULL, ia, src);
-                            ib = __shfl_sync(FULL, ib, src);
-                            g = __shfl_sync(FULL, g, src);
-                            etp = __shfl_sync(FULL, etp, src);
-                            // h and c of both rows again (the filter keeps only what its test takes)
-                            float hc[4] = {0.f, 0.f, 0.f, 0.f};
-                            for (uint32_t k = lane; k < Dp; k += 32) {
-                                const float x = sh.xn[k], ea = s.D.X[(size_t)ia * Dp + k] - x, eb = s.D.X[(size_t)ib * Dp + k] - x;
-                                hc[0] += ea * ea; hc[1] += eb * eb; hc[2] += ea * x; hc[3] += eb * x;
+                            const uint4 e = make_uint4(n, idu, __float_as_uint(sh.tA[j].w), __float_as_uint(g));
+                            if (mine && at < JOIN_TC_SAMPLES) { jq.sample[at] = e; jq.setp[at] = etp; }
+                            unsigned over = __ballot_sync(FULL, mine && at >= JOIN_TC_SAMPLES);
+                            for (; over; over &= over - 1) {   // past the record's end: here
+                                const int src = __ffs(over) - 1;
+                                SampleTally t{};
+                                sample_pair(s, __shfl_sync(FULL, e.x, src), __shfl_sync(FULL, e.y, src),
+                                            __shfl_sync(FULL, e.z, src), __uint_as_float(__shfl_sync(FULL, e.w, src)),
+                                            __shfl_sync(FULL, etp, src), lane, t);
+                                if (lane == 0) t.add(s.tc);
                             }
-#pragma unroll
-                            for (int k = 0; k < 4; ++k)
-                                for (int o = 16; o; o >>= 1) hc[k] += __shfl_xor_sync(FULL, hc[k], o);
-                            const Approx ap = approx_dist(metric, g, 0.5f * hc[0], 0.5f * hc[1], hc[2], hc[3],
-                                                          s.D.norms[ia], s.D.norms[ib], qn, etp, gam);
-                            const float apd = ap.d, ape = ap.e;
-                            const double d64 = warp_dist64(s.D, ia, ib, lane);
-                            if (lane == 0) {
-                                const double err = fabs((double)apd - d64);
-                                const double ratio = err / (double)ape;
-                                // few nodes: straight to the counters, no registers held for them
-                                atomicAdd(&s.tc->sampled, 1ull);
-                                atomicAdd(&s.tc->sum_abs, err);
-                                atomicAdd(&s.tc->sum_ratio, ratio);
-                                atomicMax(&s.tc->max_abs_bits, __float_as_uint((float)err));
-                                atomicMax(&s.tc->max_ratio_bits, __float_as_uint((float)ratio));
-                                if (d64 != 0.0) {
-                                    const double rel = err / fabs(d64);
-                                    atomicAdd(&s.tc->rel_count, 1ull);
-                                    atomicAdd(&s.tc->sum_rel, rel);
-                                    atomicMax(&s.tc->max_rel_bits, __float_as_uint((float)rel));
-                                }
-                                if (err > (double)ape) atomicAdd(&s.tc->violations, 1ull);
-                            }
+                            at += mine;
                         }
                     }
                 }
@@ -578,6 +610,20 @@ __global__ void __launch_bounds__(TC_THREADS, JOIN_TC_MAX_CTAS_PER_SM) join_tc_k
         if (comps) { atomicAdd(s.n_comps, comps); atomicAdd(&s.tc->pairs, comps); }
         if (passed) atomicAdd(&s.tc->rechecked, passed);
     }
+}
+
+// The sampled nodes' pairs, a warp each.  Evaluated where they were found, by the
+// node's own warps, the pairs of one node took about 1 ms: the tail of every
+// launch, in which the other SMs waited (200k x 96 whole build 153 -> 126 ms).
+__global__ void __launch_bounds__(256) join_sample_kernel(const __grid_constant__ BuildState s, JoinQueue jq) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t total = min(*jq.stail, JOIN_TC_SAMPLES), nw = gridDim.x * 8;
+    SampleTally t{};
+    for (uint32_t e = blockIdx.x * 8 + (threadIdx.x >> 5); e < total; e += nw) {
+        const uint4 p = jq.sample[e];
+        sample_pair(s, p.x, p.y, p.z, __uint_as_float(p.w), jq.setp[e], lane, t);
+    }
+    if (lane == 0 && t.sampled) t.add(s.tc);
 }
 
 // Phase 2: the queued pairs, 8 per warp pass: canonical FP32 distance by
@@ -694,10 +740,10 @@ cudaError_t launch_join_tc(int num_sms, int grid_insert, cudaStream_t st, const 
     occ = std::min<int>(occ, (int)((size_t)smem_sm / per_cta_smem));
     occ = std::min<int>(occ, regs_cta ? regs_sm / regs_cta : occ);
     if (occ < 1) return cudaErrorInvalidConfiguration;
-    cudaMemsetAsync(jq.tail, 0, 8, st);
-    cudaMemsetAsync(jq.work, 0, 4, st);
+    cudaMemsetAsync(jq.tail, 0, 16, st);   // tail, work, stail
     kern<<<num_sms * occ, TC_THREADS, smem, st>>>(s, s.NEWCAP + s.OLDCAP, jq, round);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    join_sample_kernel<<<num_sms * 8, 256, 0, st>>>(s, jq);
     cudaFuncSetAttribute(join_insert_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                          (int)cudaSharedmemCarveoutMaxL1);
     join_insert_kernel<<<grid_insert, 256, 0, st>>>(s, jq);
