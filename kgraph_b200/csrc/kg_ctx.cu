@@ -167,6 +167,7 @@ void kg_ctx_destroy(kg_ctx *c) {
                       &c->Xc, &c->cmeta, &c->cstats, &c->bf_rows, &c->bf_meta, &c->bf_aux, &c->bf_work};
     for (DevBuf *b : bufs) b->release();
     for (auto &b : c->build_scratch) b.release();
+    c->build_host.release();
     for (auto &b : c->rev_scratch) b.release();
     c->rseeds.release();
     kgb::router_release(c->router);

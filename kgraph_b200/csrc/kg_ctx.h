@@ -33,6 +33,21 @@ struct DevBuf {
     template <typename T> T *as() const { return reinterpret_cast<T *>(p); }
 };
 
+// Pinned host buffer that grows.
+struct HostBuf {
+    char *p = nullptr;
+    size_t bytes = 0;
+    cudaError_t reserve(size_t b) {
+        if (b <= bytes) return cudaSuccess;
+        release();
+        cudaError_t e = cudaMallocHost(reinterpret_cast<void **>(&p), b);
+        if (e == cudaSuccess) bytes = b;
+        else p = nullptr;
+        return e;
+    }
+    void release() { if (p) cudaFreeHost(p); p = nullptr; bytes = 0; }
+};
+
 struct Error {
     int code;
     std::string msg;
@@ -88,6 +103,7 @@ struct kg_ctx {
     std::vector<uint32_t> h_stage_u32;
 
     kgb::DevBuf build_scratch[25];   // NN-descent state (kg_build.cu)
+    kgb::HostBuf build_host;         // its statistics' landing place
     kgb::DevBuf rev_scratch[15];     // reverse-edge completion work space (kg_graph.cu), kept between builds
     int join_mode = KG_JOIN_AUTO;
     kgb::DevBuf tcstat;              // tensor-core join counters
