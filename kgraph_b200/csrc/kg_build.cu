@@ -569,9 +569,11 @@ __global__ void __launch_bounds__(JT_WARPS * 32, 4) join_tile_kernel(const __gri
 // is 31 instructions, where the 4-lane groups above spend two thirds of theirs on
 // exchanging partial sums and dealing tiles.  Warps share nothing, so none waits
 // for another's tiles, and a warp's loads hide behind the other warps' pairs.
-// Bound: FP32 and shared-memory issue (a broadcast 16-byte read costs four
-// cycles of the shared-memory pipe, an eighth of the pairs' FP32 instructions it
-// feeds): beyond 64 columns the tiles' reuse wins.  Whole builds, tiles against
+// Bound: FP32 issue and shared memory (a broadcast 16-byte read takes four cycles
+// of the SM's shared-memory pipe and feeds a warp eight FP32 instructions, two
+// cycles of the SM per partner row), and the gather of the rows (long-scoreboard
+// stalls); the tiles read a third as much per pair, so wide rows are theirs.
+// The line at 64 columns is the widest partner row that registers hold.  Whole builds, tiles against
 // this: 100k x 16 uniform 22.5 -> 17.1 ms, 100k x 26 32.9 -> 22.4, 200k x 48
 // mixture (K=50 L=100 S=12) 57.6 -> 45.0, 200k x 64 59.6 -> 51.2, 100k x 64
 // angular 51.0 -> 37.4.  Two partners a lane only at 16 columns: at 32 they cost
