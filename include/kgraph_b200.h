@@ -337,9 +337,7 @@ int kg_tc_assign_check(kg_ctx *ctx, const uint16_t *F, int n, int D, const uint1
  *                 scale per row (max |x_u - x_n| / 448); the margin adds each
  *                 row's exact quantisation error ||v - scale q|| (FP64) relative
  *                 to ||v||; needs d padded to a multiple of 32;
- *   KG_JOIN_AUTO  (default) the faster path measured for the build's own
- *                 workloads: KG_JOIN_FP32 (the join is bound by the locked
- *                 pool inserts, which the filter does not reduce). */
+ *   KG_JOIN_AUTO  (default) KG_JOIN_FP32. */
 enum { KG_JOIN_AUTO = 0, KG_JOIN_FP32 = 1, KG_JOIN_BF16 = 2, KG_JOIN_BF16_ALWAYS = 3, KG_JOIN_FP8 = 4,
        KG_JOIN_FP8_ALWAYS = 5 };
 int kg_set_join_precision(kg_ctx *ctx, int mode);
