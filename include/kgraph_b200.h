@@ -202,7 +202,10 @@ int kg_filter_bounds(kg_ctx *ctx, const float *queries, size_t nq, size_t q_stri
  *                         those are evaluated with the canonical FP32 distance.
  *                         No counterpart in the reference.  Memory: a BF16 copy
  *                         of the dataset (n * round_up(d, 16) * 2 bytes, and 32
- *                         bytes per row unless angular), built on first use. */
+ *                         bytes per row unless angular), built on first use, and
+ *                         a work space that the number of rows does not grow:
+ *                         queries are taken in batches of about half a gigabyte
+ *                         of intermediate results. */
 enum { KG_BRUTEFORCE_AUTO = 0, KG_BRUTEFORCE_SCAN = 1, KG_BRUTEFORCE_TENSOR = 2 };
 int kg_set_bruteforce_mode(kg_ctx *ctx, int mode);
 /* The last brute-force batch: tensor = 1 when it ran on the tensor cores;

@@ -216,13 +216,17 @@ constexpr uint32_t BF_QEXT = BF_Q * 32, BF_REXT = BF_R * 32;     // bytes of the
 constexpr uint32_t BF_MAX_ST = 6;
 constexpr size_t BF_CHUNK_BYTES = 48u << 20;
 constexpr size_t BF_SMEM = 222 * 1024;       // with the static part, within the 227 KB of a CTA
-constexpr size_t BF_BATCH = 32768;            // queries per pass over the rows (bounds the work space)
+// Queries per pass over the rows: as many as have their group maxima and candidates within
+// BF_WORK_BYTES (of a group's 4 bytes a query has up to n / 32), at most BF_BATCH.
+constexpr size_t BF_BATCH = 32768;
+constexpr size_t BF_WORK_BYTES = (size_t)512 << 20;
+constexpr uint32_t BF_MAX_GROUPS32 = 16384;   // above it groups are 128 rows
 
 struct SweepArgs {
     uint32_t n, ld, nq, nsub;
     uint32_t stages, estages;   // boxes in the ring; norm-column tiles beside it (0: angular)
     uint32_t qt, rt, rtc;    // query tiles (of nsub x 128), row tiles, row tiles per chunk
-    // sample sweep: the largest u of every `width` rows (32, 4 or 1), [group][nqp]
+    // sample sweep: the largest u of every `width` rows (128, 32, 4 or 1), [group][nqp]
     float *gmax;
     uint32_t nqp, width;
     // full sweep: per query and segment (2 per CTA that meets the query's tile) up to scap positions
@@ -414,6 +418,7 @@ __global__ void __launch_bounds__(BF_THREADS, 1)
                 const uint32_t base = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + acc * BF_R + 128 * half;
                 const uint32_t qi = (tq * nsub + s) * BF_Q + row32;
                 uint32_t buf[2][32];
+                float m128 = -INFINITY;   // sample sweep: over this warp's columns of the tile
                 tc::tmem_ld32_issue(base, buf[0]);
 #pragma unroll
                 for (int part = 0; part < 4; ++part) {
@@ -444,7 +449,9 @@ __global__ void __launch_bounds__(BF_THREADS, 1)
                                     if (wd == 4) o[(size_t)(k / 4) * a.nqp] = f;
                                     m = fmaxf(m, f);
                                 }
-                                if (wd == 32) *o = m;
+                                m128 = fmaxf(m128, m);
+                                if (wd == 32 || (wd == 128 && part == 3)) *o = m128;
+                                if (wd == 32) m128 = -INFINITY;
                             }
                         }
                     } else {
@@ -788,8 +795,29 @@ int bruteforce_prepare(kg_ctx *ctx) {
     return KG_OK;
 }
 
-// One pass over the rows for at most BF_BATCH queries.
-static int bruteforce_batch(kg_ctx *ctx, const float *Q, uint32_t q_ld, uint32_t nq, uint32_t K, float epsilon,
+// The sample sweep's rows and groups, the candidates a query has room for, and
+// how many queries take one pass.
+struct SweepPlan {
+    uint32_t cap, ns, width;
+    size_t batch;
+    SweepPlan(uint32_t n, uint32_t K) : cap(std::max<uint32_t>(1024, 8 * K)) {
+        // A share of the rows that leaves about K / share candidates per query, at most half of `cap`;
+        // groups of 32 rows where that makes at least 8 K of them, else smaller ones, so that few of the
+        // K nearest sampled rows share a group.
+        const uint32_t share = K <= 2 ? 8 : K <= 24 ? 16 : K <= 64 ? 8 : 4;
+        ns = n / share / BF_R * BF_R;
+        if (ns < 4096) ns = n;
+        width = ns / 32 >= 8 * K ? 32 : ns / 4 >= 8 * K ? 4 : 1;
+        if (ns / 32 > BF_MAX_GROUPS32) width = 128;
+        const size_t per = (size_t)(ns / width + BF_R) * 4 + (size_t)8 * cap;
+        batch = std::min(BF_BATCH, std::max<size_t>(BF_WORK_BYTES / per, 32));
+        const size_t tile = batch >= 2 * BF_Q ? 2 * BF_Q : 32;   // whole tiles of queries where there are some
+        batch = batch / tile * tile;
+    }
+};
+
+// One pass over the rows for at most p.batch queries.
+static int bruteforce_batch(kg_ctx *ctx, const SweepPlan &p, const float *Q, uint32_t q_ld, uint32_t nq, uint32_t K, float epsilon,
                             uint32_t *out_ids, float *out_d, uint32_t *out_cnt, float *out_cost, uint32_t out_ld,
                             unsigned long long *stats, unsigned long long *work) {
     const uint32_t n = ctx->n, ld = ctx->ld;
@@ -808,14 +836,7 @@ static int bruteforce_batch(kg_ctx *ctx, const float *Q, uint32_t q_ld, uint32_t
     const uint32_t qt = (nq + nsub * BF_Q - 1) / (nsub * BF_Q), rt = (n + BF_R - 1) / BF_R;
     const uint32_t chunks = (uint32_t)(((size_t)n * ld * 2 + BF_CHUNK_BYTES - 1) / BF_CHUNK_BYTES);
     const uint32_t rtc = (rt + chunks - 1) / chunks;
-    const uint32_t cap = std::max<uint32_t>(1024, 8 * K);
-    // The sample: a share of the rows that leaves about K / share candidates per query, at most half
-    // of `cap`; groups of 32 rows where that makes at least 8 K of them, else smaller ones, so that
-    // few of the K nearest sampled rows share a group.
-    const uint32_t share = K <= 2 ? 8 : K <= 24 ? 16 : K <= 64 ? 8 : 4;
-    uint32_t ns = n / share / BF_R * BF_R;
-    if (ns < 4096) ns = n;
-    const uint32_t width = ns / 32 >= 8 * K ? 32 : ns / 4 >= 8 * K ? 4 : 1;
+    const uint32_t cap = p.cap, ns = p.ns, width = p.width;
     const uint32_t srt = (ns + BF_R - 1) / BF_R, groups = (ns + width - 1) / width;
     const uint32_t fold = (groups + BF_GROUPS - 1) / BF_GROUPS, G = (groups + fold - 1) / fold;
     const uint32_t nqp = (nq + 31) / 32 * 32;
@@ -838,8 +859,8 @@ static int bruteforce_batch(kg_ctx *ctx, const float *Q, uint32_t q_ld, uint32_t
     const size_t need = pad((size_t)nq * ld * 2) + pad((size_t)nq * 16) + pad((size_t)srt * (BF_R / width) * nqp * 4) +
                         pad((size_t)nq * 4) + pad((size_t)nq * nseg * scap * 4) + pad((size_t)nq * nseg * 4);
     if ((e = ctx->bf_work.reserve(need)) != cudaSuccess) return cuda_fail(ctx, e, "alloc brute force");
-    char *p = ctx->bf_work.as<char>();
-    auto carve = [&](size_t bytes) { char *q = p; p += pad(bytes); return q; };
+    char *at = ctx->bf_work.as<char>();
+    auto carve = [&](size_t bytes) { char *q = at; at += pad(bytes); return q; };
     __nv_bfloat16 *Qb = reinterpret_cast<__nv_bfloat16 *>(carve((size_t)nq * ld * 2));
     float4 *qmeta = reinterpret_cast<float4 *>(carve((size_t)nq * 16));
     float *gmax = reinterpret_cast<float *>(carve((size_t)srt * (BF_R / width) * nqp * 4));
@@ -898,9 +919,10 @@ int bruteforce_tc(kg_ctx *ctx, const float *Q, uint32_t q_ld, uint32_t nq, uint3
     unsigned long long *stats = reinterpret_cast<unsigned long long *>(ctx->bf_aux.as<char>() + (size_t)ctx->ld * 12 + 64);
     cudaMemsetAsync(stats, 0, 16, ctx->stream);
     ctx->bf_stats_dev = stats;
-    for (size_t q0 = 0; q0 < nq; q0 += BF_BATCH) {
-        const uint32_t m = (uint32_t)std::min<size_t>(BF_BATCH, nq - q0);
-        const int r = bruteforce_batch(ctx, Q + q0 * q_ld, q_ld, m, K, epsilon, out_ids + q0 * out_ld,
+    const SweepPlan p(ctx->n, K);
+    for (size_t q0 = 0; q0 < nq; q0 += p.batch) {
+        const uint32_t m = (uint32_t)std::min<size_t>(p.batch, nq - q0);
+        const int r = bruteforce_batch(ctx, p, Q + q0 * q_ld, q_ld, m, K, epsilon, out_ids + q0 * out_ld,
                                        out_d ? out_d + q0 * out_ld : nullptr, out_cnt + q0,
                                        out_cost ? out_cost + q0 : nullptr, out_ld, stats, work);
         if (r != KG_OK) return r;
