@@ -210,8 +210,10 @@ enum { KG_BRUTEFORCE_AUTO = 0, KG_BRUTEFORCE_SCAN = 1, KG_BRUTEFORCE_TENSOR = 2 
 int kg_set_bruteforce_mode(kg_ctx *ctx, int mode);
 /* The last brute-force batch: tensor = 1 when it ran on the tensor cores;
  * candidates = rows evaluated in FP32 over all queries; full_scans = queries
- * whose candidates exceeded the per-query capacity (max(1024, 8 K)) and were
- * scanned in full instead. */
+ * that were scanned in full instead: those without a finite margin (a NaN, an
+ * infinity or, angular, a zero norm in the query, or a data set whose rows are
+ * all zero) and those whose margin admits more rows than a query has room for
+ * (max(2048, 16 K), and half of that in one part of the rows). */
 typedef struct {
     int tensor;
     unsigned long long candidates, full_scans;

@@ -32,8 +32,15 @@
 //      the sampled share;
 //   5. one warp per query evaluates its candidates with the canonical FP32
 //      distance and keeps the K smallest by (distance, id) within epsilon --
-//      the reference's list.  A query with more candidates than its room is
-//      scanned in full on the CUDA cores instead (counted in the statistics).
+//      the reference's list;
+//   6. a query with more candidates than its room goes through 2 to 5 once more,
+//      now with all rows as the sample, which leaves about K candidates instead
+//      of K over the share, and with twice the room.  Only where the margin alone
+//      admits more rows than that is it scanned in full on the CUDA cores
+//      (counted in the statistics), which takes a warp 37 ms for 200k rows of
+//      128: 1,000 queries, K = 10, on a float mixture of that size with centres
+//      twice the spread, 605 of them with too many candidates from the sample,
+//      34 ms without this step, 0.96 ms with it.
 //
 // All tensor-core waits are bounded: a wait that runs out raises
 // ERR_TC_TIMEOUT, waits (bounded) for what is in flight, frees the CTA's TMEM
@@ -142,12 +149,13 @@ __global__ void prep_rows_kernel(DataView D, const float *mu, uint64_t inv, __nv
 
 // One warp per query: the same centring and rounding, and the canonical norm
 // term of the query (the search kernel's computation: python-api.cpp:98-101).
-__global__ void prep_queries_kernel(DataView D, const float *mu, const float *Q, uint32_t q_ld, uint32_t nq,
-                                    __nv_bfloat16 *Qb, float4 *qmeta) {
+// `map`, if given, holds the queries' rows.
+__global__ void prep_queries_kernel(DataView D, const float *mu, const float *Q, uint32_t q_ld, const uint32_t *map,
+                                    uint32_t nq, __nv_bfloat16 *Qb, float4 *qmeta) {
     const int lane = threadIdx.x & 31;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t qi = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; qi < nq; qi += warps) {
-        const float *q = Q + (size_t)qi * q_ld;
+        const float *q = Q + (size_t)(map ? map[qi] : qi) * q_ld;
         double e2 = 0.0, v2 = 0.0;
         for (uint32_t j = lane; j < D.ld; j += 32) {
             const float xc = j < D.d ? __fsub_rn(q[j], mu[j]) : 0.f;
@@ -599,10 +607,13 @@ __device__ __forceinline__ float key_dist(unsigned long long k) {
 }
 
 // One warp per query: canonical FP32 distances of the candidates, then the K
-// smallest by (distance, id) within epsilon; a query whose candidates
-// overflowed is scanned in full.
-__global__ void __launch_bounds__(256) bf_recheck_kernel(DataView D, const float *Q, uint32_t q_ld, uint32_t nq,
-                                                         uint32_t K, float epsilon, const uint32_t *cand,
+// smallest by (distance, id) within epsilon.  A query whose candidates
+// overflowed is noted in `again` (its row; the count in stats[2]) or, without
+// one, scanned in full; one without a margin is scanned in full.  The queries'
+// rows are map[0 .. nq) or, without a map, q0 .. q0 + nq - 1.
+__global__ void __launch_bounds__(256) bf_recheck_kernel(DataView D, const float *Q, uint32_t q_ld, uint32_t q0,
+                                                         const uint32_t *map, uint32_t nq, uint32_t K, float epsilon,
+                                                         const float *thresh, uint32_t *again, const uint32_t *cand,
                                                          const uint32_t *cand_n, uint32_t nseg, uint32_t scap,
                                                          uint64_t mult, uint32_t cap, uint32_t *out_ids,
                                                          float *out_d, uint32_t *out_cnt, float *out_cost,
@@ -612,10 +623,11 @@ __global__ void __launch_bounds__(256) bf_recheck_kernel(DataView D, const float
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t qi = blockIdx.x * (blockDim.x >> 5) + w;
     if (qi >= nq) return;   // whole warps
+    const size_t row = map ? map[qi] : q0 + qi;
     float *q = reinterpret_cast<float *>(rsm) + (size_t)w * D.ld;
     unsigned long long *keys = reinterpret_cast<unsigned long long *>(rsm + (size_t)(blockDim.x >> 5) * D.ld * 4) +
                                (size_t)w * cap;
-    for (uint32_t x = lane; x < D.ld; x += 32) q[x] = x < D.d ? Q[(size_t)qi * q_ld + x] : 0.f;
+    for (uint32_t x = lane; x < D.ld; x += 32) q[x] = x < D.d ? Q[row * q_ld + x] : 0.f;
     __syncwarp();
     float qn = 0.f;
     if (D.metric != METRIC_L2SQR) qn = norm_term(group4_raw(q, q, D.d, METRIC_EUCLIDEAN, lane & 3, FULL), D.metric);
@@ -638,6 +650,10 @@ __global__ void __launch_bounds__(256) bf_recheck_kernel(DataView D, const float
         const uint32_t *src = cand + ((size_t)qi * nseg + s0 + lane) * scap;
         for (uint32_t i = 0; i < k; ++i) ids[nc + end - k + i] = (uint32_t)(src[i] * mult % D.n);   // position p holds row p * mult mod n
         nc += sum;
+    }
+    if (full && again && thresh[qi] < INFINITY) {
+        if (lane == 0) again[atomicAdd(stats + 2, 1ull)] = (uint32_t)row;
+        return;
     }
     __syncwarp();
     const uint32_t total = full ? D.n : nc;
@@ -694,8 +710,8 @@ __global__ void __launch_bounds__(256) bf_recheck_kernel(DataView D, const float
     __syncwarp();
     // K rounds of the warp's smallest remaining key
     const uint32_t cnt = min(K, nkeys);
-    uint32_t *oi = out_ids + (size_t)qi * out_ld;
-    float *od = out_d ? out_d + (size_t)qi * out_ld : nullptr;
+    uint32_t *oi = out_ids + row * out_ld;
+    float *od = out_d ? out_d + row * out_ld : nullptr;
     for (uint32_t k = 0; k < cnt; ++k) {
         unsigned long long mn = ~0ull;
         uint32_t at = 0;
@@ -716,8 +732,8 @@ __global__ void __launch_bounds__(256) bf_recheck_kernel(DataView D, const float
         __syncwarp();
     }
     if (lane == 0) {
-        out_cnt[qi] = cnt;
-        if (out_cost) out_cost[qi] = 1.0f;   // kgraph.cpp:428-431
+        out_cnt[row] = cnt;
+        if (out_cost) out_cost[row] = 1.0f;   // kgraph.cpp:428-431
         atomicAdd(stats + 0, (unsigned long long)(full ? 0u : nc));
         if (full) atomicAdd(stats + 1, 1ull);
         if (work) atomicAdd(work, (unsigned long long)total);
@@ -796,28 +812,30 @@ int bruteforce_prepare(kg_ctx *ctx) {
 }
 
 // The sample sweep's rows and groups, the candidates a query has room for, and
-// how many queries take one pass.
+// how many queries take one pass.  `all`: for queries that come a second time,
+// all rows are the sample.
 struct SweepPlan {
     uint32_t cap, ns, width;
     size_t batch;
-    SweepPlan(uint32_t n, uint32_t K) : cap(std::max<uint32_t>(1024, 8 * K)) {
+    SweepPlan(uint32_t n, uint32_t K, bool all) : cap((all ? 2 : 1) * std::max<uint32_t>(1024, 8 * K)) {
         // A share of the rows that leaves about K / share candidates per query, at most half of `cap`;
         // groups of 32 rows where that makes at least 8 K of them, else smaller ones, so that few of the
         // K nearest sampled rows share a group.
-        const uint32_t share = K <= 2 ? 8 : K <= 24 ? 16 : K <= 64 ? 8 : 4;
+        const uint32_t share = all ? 1 : K <= 2 ? 8 : K <= 24 ? 16 : K <= 64 ? 8 : 4;
         ns = n / share / BF_R * BF_R;
-        if (ns < 4096) ns = n;
+        if (ns < 4096 || share == 1) ns = n;
         width = ns / 32 >= 8 * K ? 32 : ns / 4 >= 8 * K ? 4 : 1;
         if (ns / 32 > BF_MAX_GROUPS32) width = 128;
-        const size_t per = (size_t)(ns / width + BF_R) * 4 + (size_t)8 * cap;
+        const size_t per = (size_t)(ns / width + BF_R) * 4 + (size_t)(all ? 24 : 8) * cap;
         batch = std::min(BF_BATCH, std::max<size_t>(BF_WORK_BYTES / per, 32));
         const size_t tile = batch >= 2 * BF_Q ? 2 * BF_Q : 32;   // whole tiles of queries where there are some
         batch = batch / tile * tile;
     }
 };
 
-// One pass over the rows for at most p.batch queries.
-static int bruteforce_batch(kg_ctx *ctx, const SweepPlan &p, const float *Q, uint32_t q_ld, uint32_t nq, uint32_t K, float epsilon,
+// One pass over the rows for at most p.batch queries: rows q0 .. q0 + nq - 1, or map[0 .. nq).
+static int bruteforce_batch(kg_ctx *ctx, const SweepPlan &p, const float *Q, uint32_t q_ld, uint32_t q0,
+                            const uint32_t *map, uint32_t nq, uint32_t K, float epsilon, uint32_t *again,
                             uint32_t *out_ids, float *out_d, uint32_t *out_cnt, float *out_cost, uint32_t out_ld,
                             unsigned long long *stats, unsigned long long *work) {
     const uint32_t n = ctx->n, ld = ctx->ld;
@@ -843,7 +861,8 @@ static int bruteforce_batch(kg_ctx *ctx, const SweepPlan &p, const float *Q, uin
     const uint32_t grid1 = (uint32_t)std::min<uint64_t>(ctx->num_sms, (uint64_t)qt * rtc);
     const uint32_t grid0 = (uint32_t)std::min<uint64_t>(ctx->num_sms, (uint64_t)qt * srt);
     // segments of candidates: two (column halves) per CTA that meets a query tile, each with room for
-    // twice its even share (the spread order deals the candidates out evenly)
+    // twice its even share (the spread order deals the candidates out evenly); the queries that come a
+    // second time get twice the share of the CTA that meets most of their tile
     uint32_t nseg = 1;
     for (uint32_t q = 0; q < qt; ++q) {
         const uint32_t b0 = sweep_first_cta(q, qt, rtc, grid1);
@@ -853,7 +872,9 @@ static int bruteforce_batch(kg_ctx *ctx, const SweepPlan &p, const float *Q, uin
         nseg = std::max(nseg, b1 - b0 + 1);
     }
     nseg *= 2;
-    const uint32_t scap = std::min<uint32_t>(cap, std::max<uint32_t>(128, 2 * cap / nseg));
+    uint32_t even = 2 * cap / nseg;
+    if (!again) even = (uint32_t)std::min<uint64_t>(cap, (uint64_t)cap * ((uint64_t)qt * rtc / grid1 + 1) / rtc);
+    const uint32_t scap = std::min<uint32_t>(cap, std::max<uint32_t>(128, even));
     cudaError_t e;
     auto pad = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t need = pad((size_t)nq * ld * 2) + pad((size_t)nq * 16) + pad((size_t)srt * (BF_R / width) * nqp * 4) +
@@ -871,7 +892,7 @@ static int bruteforce_batch(kg_ctx *ctx, const SweepPlan &p, const float *Q, uin
     const DataView D{ctx->X.as<float>(), ctx->norms.as<float>(), n, ctx->d, ld, ctx->metric};
     const float *mu = reinterpret_cast<const float *>(ctx->bf_aux.as<double>() + ld);
     prep_queries_kernel<<<std::max<uint32_t>(1, std::min<uint32_t>((nq + 7) / 8, ctx->num_sms * 8)), 256, 0, st>>>(
-        D, mu, Q, q_ld, nq, Qb, qmeta);
+        D, mu, map ? Q : Q + (size_t)q0 * q_ld, q_ld, map, nq, Qb, qmeta);
     CUtensorMap mQ, mX, mE;
     if (!tc_bf16_map(&mQ, Qb, ld, nq, ld, 64, BF_Q) || !tc_bf16_map(&mX, ctx->bf_rows.p, ld, n, ld, 64, BF_R))
         return set_error(ctx, KG_E_CUDA, "brute force: tensor map");
@@ -907,24 +928,40 @@ static int bruteforce_batch(kg_ctx *ctx, const SweepPlan &p, const float *Q, uin
     if ((e = cudaFuncSetAttribute(bf_recheck_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsmem)) !=
         cudaSuccess)
         return cuda_fail(ctx, e, "brute-force recheck attributes");
-    bf_recheck_kernel<<<(nq + wpb - 1) / wpb, wpb * 32, rsmem, st>>>(D, Q, q_ld, nq, K, epsilon, cand, cand_n, nseg, scap, ctx->bf_mult, cap,
-                                                                     out_ids, out_d, out_cnt, out_cost, out_ld, stats, work);
+    bf_recheck_kernel<<<(nq + wpb - 1) / wpb, wpb * 32, rsmem, st>>>(D, Q, q_ld, q0, map, nq, K, epsilon, thresh, again,
+                                                                     cand, cand_n, nseg, scap, ctx->bf_mult, cap, out_ids,
+                                                                     out_d, out_cnt, out_cost, out_ld, stats, work);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e, "brute-force launch");
     return KG_OK;
 }
 
 int bruteforce_tc(kg_ctx *ctx, const float *Q, uint32_t q_ld, uint32_t nq, uint32_t K, float epsilon, uint32_t *out_ids,
                   float *out_d, uint32_t *out_cnt, float *out_cost, uint32_t out_ld, unsigned long long *work) {
-    // candidates rechecked, queries scanned in full (read by the caller after its sync); behind the mean
+    cudaError_t e;
+    if ((e = ctx->bf_again.reserve((size_t)nq * 4)) != cudaSuccess) return cuda_fail(ctx, e, "alloc brute force");
+    // candidates rechecked, queries scanned in full, queries to come again (read by the caller after its
+    // sync); behind the mean
     unsigned long long *stats = reinterpret_cast<unsigned long long *>(ctx->bf_aux.as<char>() + (size_t)ctx->ld * 12 + 64);
-    cudaMemsetAsync(stats, 0, 16, ctx->stream);
+    cudaMemsetAsync(stats, 0, 24, ctx->stream);
     ctx->bf_stats_dev = stats;
-    const SweepPlan p(ctx->n, K);
+    const SweepPlan p(ctx->n, K, false);
     for (size_t q0 = 0; q0 < nq; q0 += p.batch) {
-        const uint32_t m = (uint32_t)std::min<size_t>(p.batch, nq - q0);
-        const int r = bruteforce_batch(ctx, p, Q + q0 * q_ld, q_ld, m, K, epsilon, out_ids + q0 * out_ld,
-                                       out_d ? out_d + q0 * out_ld : nullptr, out_cnt + q0,
-                                       out_cost ? out_cost + q0 : nullptr, out_ld, stats, work);
+        const int r = bruteforce_batch(ctx, p, Q, q_ld, (uint32_t)q0, nullptr, (uint32_t)std::min<size_t>(p.batch, nq - q0),
+                                       K, epsilon, ctx->bf_again.as<uint32_t>(), out_ids, out_d, out_cnt, out_cost,
+                                       out_ld, stats, work);
+        if (r != KG_OK) return r;
+    }
+    return KG_OK;
+}
+
+int bruteforce_again(kg_ctx *ctx, const float *Q, uint32_t q_ld, uint32_t count, uint32_t K, float epsilon,
+                     uint32_t *out_ids, float *out_d, uint32_t *out_cnt, float *out_cost, uint32_t out_ld,
+                     unsigned long long *work) {
+    const SweepPlan p(ctx->n, K, true);
+    for (size_t i = 0; i < count; i += p.batch) {
+        const int r = bruteforce_batch(ctx, p, Q, q_ld, 0, ctx->bf_again.as<uint32_t>() + i,
+                                       (uint32_t)std::min<size_t>(p.batch, count - i), K, epsilon, nullptr, out_ids,
+                                       out_d, out_cnt, out_cost, out_ld, ctx->bf_stats_dev, work);
         if (r != KG_OK) return r;
     }
     return KG_OK;

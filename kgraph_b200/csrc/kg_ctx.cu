@@ -164,7 +164,8 @@ void kg_ctx_destroy(kg_ctx *c) {
                       &c->visited, &c->qbuf, &c->kbuf, &c->pbuf, &c->seeds, &c->seed_index, &c->init_ids,
                       &c->out_ids, &c->out_d, &c->out_cnt, &c->out_cost, &c->tcstat, &c->joinq, &c->joinaux, &c->joinb,
                       &c->offer_lin, &c->offer_grp, &c->offer_aux, &c->offer_scan,
-                      &c->Xc, &c->cmeta, &c->cstats, &c->bf_rows, &c->bf_meta, &c->bf_aux, &c->bf_work};
+                      &c->Xc, &c->cmeta, &c->cstats, &c->bf_rows, &c->bf_meta, &c->bf_aux, &c->bf_work,
+                      &c->bf_again};
     for (DevBuf *b : bufs) b->release();
     for (auto &b : c->build_scratch) b.release();
     c->build_host.release();
@@ -533,16 +534,26 @@ int search_locked(kg_ctx *ctx, const float *queries, size_t nq, size_t q_stride_
     ctx->last_shape = sh;   // the shape as launched: its query tile and whether the compact pool ran
     ctx->last_shape.warps_per_block = use_tc_bf ? 0u : a.warps_per_block;
     ctx->last_shape.compact = (!use_tc_bf && search_uses_compact(a, sh)) ? 1u : 0u;
-    cudaEventRecord(ctx->ev1, ctx->stream);
-    unsigned long long bf_h[2] = {0, 0};
-    if (use_tc_bf) cudaMemcpyAsync(bf_h, ctx->bf_stats_dev, 16, cudaMemcpyDeviceToHost, ctx->stream);
-
-    if (!ids_dev) cudaMemcpyAsync(ids, a.out_ids, Q * out_ld * 4, cudaMemcpyDeviceToHost, ctx->stream);
-    if (dists && !d_dev) cudaMemcpyAsync(dists, a.out_dists, Q * out_ld * 4, cudaMemcpyDeviceToHost, ctx->stream);
-    if (!c_dev) cudaMemcpyAsync(counts, a.out_count, Q * 4, cudaMemcpyDeviceToHost, ctx->stream);
-    if (costs && !cost_dev) cudaMemcpyAsync(costs, a.out_cost, Q * 4, cudaMemcpyDeviceToHost, ctx->stream);
-    cudaMemcpyAsync(ctx->last_work, a.work, 32, cudaMemcpyDeviceToHost, ctx->stream);
-    if ((e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) return cuda_fail(ctx, e, "search");
+    unsigned long long bf_h[3] = {0, 0, 0};
+    auto finish = [&]() {
+        cudaEventRecord(ctx->ev1, ctx->stream);
+        if (use_tc_bf) cudaMemcpyAsync(bf_h, ctx->bf_stats_dev, 24, cudaMemcpyDeviceToHost, ctx->stream);
+        if (!ids_dev) cudaMemcpyAsync(ids, a.out_ids, Q * out_ld * 4, cudaMemcpyDeviceToHost, ctx->stream);
+        if (dists && !d_dev) cudaMemcpyAsync(dists, a.out_dists, Q * out_ld * 4, cudaMemcpyDeviceToHost, ctx->stream);
+        if (!c_dev) cudaMemcpyAsync(counts, a.out_count, Q * 4, cudaMemcpyDeviceToHost, ctx->stream);
+        if (costs && !cost_dev) cudaMemcpyAsync(costs, a.out_cost, Q * 4, cudaMemcpyDeviceToHost, ctx->stream);
+        cudaMemcpyAsync(ctx->last_work, a.work, 32, cudaMemcpyDeviceToHost, ctx->stream);
+        return cudaStreamSynchronize(ctx->stream);
+    };
+    if ((e = finish()) != cudaSuccess) return cuda_fail(ctx, e, "search");
+    if (bf_h[2]) {   // brute-force queries with more candidates than their room, known only now
+        int br = check_device_error(ctx, "search");
+        if (br == KG_OK)
+            br = bruteforce_again(ctx, a.Q, a.q_ld, (uint32_t)bf_h[2], params->K, params->epsilon, a.out_ids,
+                                  a.out_dists, a.out_count, a.out_cost, (uint32_t)out_ld, a.work);
+        if (br != KG_OK) return br;
+        if ((e = finish()) != cudaSuccess) return cuda_fail(ctx, e, "search");
+    }
     cudaEventElapsedTime(&ctx->last_search_ms, ctx->ev0, ctx->ev1);
     if (use_tc_bf) {
         ctx->last_bf.tensor = 1;

@@ -114,8 +114,8 @@ struct kg_ctx {
     bool join_tile = true;            // FP32 join with each node's lists staged in shared memory
     kg_join_stats last_join{};
     // tensor-core brute force (kg_bruteforce.cu): BF16 centred rows in the spread order (position p holds
-    // row p * bf_mult mod n), their norm columns, mean + extents, work space
-    kgb::DevBuf bf_rows, bf_meta, bf_aux, bf_work;
+    // row p * bf_mult mod n), their norm columns, mean + extents, work space, queries to come a second time
+    kgb::DevBuf bf_rows, bf_meta, bf_aux, bf_work, bf_again;
     uint64_t bf_data_version = ~0ull;
     float bf_ext[4] = {0, 0, 0, 0};
     uint64_t bf_mult = 1;
