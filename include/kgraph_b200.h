@@ -394,7 +394,9 @@ int kg_join_merge_check(kg_ctx *ctx, unsigned n, unsigned L, unsigned K, float *
  * is also evaluated in FP64: sampled pairs, the BF16 tile distance's absolute
  * and relative error against FP64 (max, mean) and the error as a fraction of
  * the margin (max, mean; < 1 means the filter was safe); violations = sampled
- * or rechecked pairs whose error exceeded the margin. */
+ * pairs whose error exceeded the margin, whose lower bound in the filter's own
+ * test lay above their distance (FP64 or canonical), or that it skipped although
+ * their canonical distance is not above both endpoints' radii. */
 typedef struct {
     int mode;
     unsigned long long pairs, rechecked, sampled, violations;

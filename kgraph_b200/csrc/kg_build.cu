@@ -1579,11 +1579,11 @@ extern "C" int kg_build(kg_ctx *ctx, const kg_index_params *params, kg_index_inf
     if (use_tc) {
         // (x, y, node) entries for one round's pairs; rounds are cut to fit
         qcap = std::max<uint64_t>(64ull << 20, 4 * join_tc_node_max(s));
-        if ((e = ctx->joinq.reserve(JOIN_TC_SAMPLES * 20ull + qcap * 12 + 64)) != cudaSuccess) return cuda_fail(ctx, e, "alloc join queue");
+        if ((e = ctx->joinq.reserve(JOIN_TC_SAMPLES * 32ull + qcap * 12 + 64)) != cudaSuccess) return cuda_fail(ctx, e, "alloc join queue");
         if ((e = ctx->joinaux.reserve((n + 1) * 16)) != cudaSuccess) return cuda_fail(ctx, e, "alloc join queue");
         jq.sample = ctx->joinq.as<uint4>();
-        jq.setp = reinterpret_cast<float *>(jq.sample + JOIN_TC_SAMPLES);
-        jq.x = reinterpret_cast<uint32_t *>(jq.setp + JOIN_TC_SAMPLES);
+        jq.filter = reinterpret_cast<float4 *>(jq.sample + JOIN_TC_SAMPLES);
+        jq.x = reinterpret_cast<uint32_t *>(jq.filter + JOIN_TC_SAMPLES);
         jq.y = jq.x + qcap;
         jq.n = jq.y + qcap;
         jq.tail = reinterpret_cast<unsigned long long *>(jq.n + qcap + (qcap & 1));

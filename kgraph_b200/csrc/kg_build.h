@@ -72,8 +72,8 @@ struct JoinQueue {
     unsigned long long *tail;
     uint32_t *work;      // claim counter within a round
     uint32_t *stail;     // sampled pairs of the round (recorded while below JOIN_TC_SAMPLES)
-    uint4 *sample;       // {node, rows, Gram entry} of a sampled pair, and its product error
-    float *setp;
+    uint4 *sample;       // {node, rows, Gram entry} of a sampled pair, and the filter's decision (sample_pair)
+    float4 *filter;
     uint32_t *bounds;    // round boundaries (node ids)
 };
 constexpr int JOIN_TC_MAX_CTAS_PER_SM = 6;

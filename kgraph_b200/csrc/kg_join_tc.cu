@@ -31,16 +31,19 @@
 //      above BOTH endpoints' radius cannot pass the reference's unlocked
 //      radius test (kgraph.cpp:725, radii only shrink during a join), so it is
 //      skipped.  Every other pair is recomputed with the canonical FP32
-//      distance and goes through the same locked insert as the CUDA-core join:
-//      every heap insert, ordering and stored distance is decided in FP32.
+//      distance and offered as the CUDA-core join offers its pairs (to the
+//      record of deferred inserts, or inserted under the pools' locks): every
+//      insert, ordering and stored distance is decided in FP32.
 //
 // The margin E bounds |approx - exact| + |canonical FP32 - exact| with a
 // factor 2 of slack: BF16 rounding of both operands (2^-8 + 2^-17 relative to
 // |x_u - x_n| |x_j - x_n|), FP32 accumulation of D products (up to 2^-23 each),
 // the FP32 centering and norm sums, and the canonical distance's own error
-// (D + 4 ulps of the uncentered norms).  A sample of nodes (about 1 in 2048)
-// also evaluates every pair in FP64 and records the tile error and its ratio
-// to E (JoinTcStats), so the bound is checked on every run.
+// (D + 4 ulps of the uncentered norms).  On a sample of nodes (about 1 in 2048)
+// every pair is also evaluated in FP64 and in canonical FP32: the tile error and
+// its ratio to E are recorded (JoinTcStats), and a pair whose lower bound, as the
+// test itself formed it, lies above its distance, or that was skipped although a
+// pool would take it, is a violation.
 //
 // All waits are bounded: the MMA completion barrier gives up after ~1 s,
 // raises ERR_TC_TIMEOUT and the CTA drains, frees its TMEM and returns.
@@ -51,6 +54,7 @@
 #include <cuda_fp8.h>
 #include "kg_build.h"
 #include "kg_insert.cuh"
+#include "kg_join_filter.h"
 #include "kg_tc.cuh"
 
 namespace kgb {
@@ -63,6 +67,9 @@ constexpr uint32_t TC_REST = TC_M - TC_N;   // partners per tile besides the col
 constexpr uint32_t TC_TMEM_COLS = 32;
 constexpr long long TC_WAIT_CYCLES = 2000000000ll;
 constexpr uint32_t TC_CLAIM = 8;         // nodes claimed per CTA at a time
+
+static_assert((int)FILTER_EUCLIDEAN == METRIC_EUCLIDEAN && (int)FILTER_ANGULAR == METRIC_ANGULAR &&
+              (int)FILTER_L2SQR == METRIC_L2SQR, "FilterMetric");
 
 __device__ __forceinline__ bool sampled_node(uint32_t n) { return ((n * 0x9E3779B1u) >> 21) == 0; }
 
@@ -129,9 +136,12 @@ struct SampleTally {
 };
 
 // Whole warp: the error of the approximate distance of rows ia and ib of node
-// n's lists (Gram entry g, product error etp) against FP64.
-__device__ __noinline__ void sample_pair(const BuildState &s, uint32_t n, uint32_t ia, uint32_t ib, float g, float etp,
+// n's lists (Gram entry g) against FP64, and the filter's own decision against
+// the distances.  f: {product error, the filter's lower bound, the larger radius as
+// it held it, 1 where it skipped the pair}.
+__device__ __noinline__ void sample_pair(const BuildState &s, uint32_t n, uint32_t ia, uint32_t ib, float g, float4 f,
                                          int lane, SampleTally &t) {
+    const float etp = f.x;
     const uint32_t Dp = s.D.ld;
     const float gam = (float)(s.D.d + 4) * 5.9605e-8f;
     const float *xn = s.D.X + (size_t)n * Dp;
@@ -148,6 +158,7 @@ __device__ __noinline__ void sample_pair(const BuildState &s, uint32_t n, uint32
     }
     const Approx ap = approx_dist(s.D.metric, g, 0.5f * hc[0], 0.5f * hc[1], hc[2], hc[3], s.D.norms[ia], s.D.norms[ib],
                                   qn, etp, gam);
+    const float dc = pair_dist(s.D, ia, ib, lane & 3, FULL);
     const double d64 = warp_dist64(s.D, ia, ib, lane), err = fabs((double)ap.d - d64), ratio = err / (double)ap.e;
     ++t.sampled;
     t.sum_abs += err;
@@ -160,7 +171,9 @@ __device__ __noinline__ void sample_pair(const BuildState &s, uint32_t n, uint32
         t.sum_rel += rel;
         t.max_rel = max(t.max_rel, __float_as_uint((float)rel));
     }
-    if (err > (double)ap.e) ++t.violations;
+    const bool wrong = filter_wrong((FilterMetric)s.D.metric, f.y, f.w != 0.f, f.z, s.D.norms ? s.D.norms[ia] : 0.f,
+                                    s.D.norms ? s.D.norms[ib] : 0.f, d64, dc);
+    if (err > (double)ap.e || wrong) ++t.violations;
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -177,28 +190,11 @@ struct TcShared {
 };
 constexpr uint32_t TC_PAD = 16;   // the epilogue reads columns 16 at a time, past the last row
 
-// The filter's test, approx d - E > max radius, without a square root or a
-// division per pair: both sides times the denominator (angular), the margin's
-// terms split into one part per row, |x_u - x_n| |x_j - x_n| = s_u s_j with
-// s = sqrt(2 h) per row.
-// euclidean and l2sqr (halved): A_u + A_j - g - 2 et s_u s_j > max radius;
-// angular, full = g + A_u + A_j, w = n_u n_j:
-//   -full - 2 et s_u s_j - C_u - C_j - 2 gam w - 4 gam |full| - 4.8e-7 |g|
-//   > max radius (w + FLT_EPSILON).
-// Its rounding is a few parts in 2^24 of the same terms, inside the factor 2 of E.
-// h = |x_u - x_n|^2 / 2, c = (x_u - x_n) . x_n, qn = |x_n|^2.
 __device__ __forceinline__ void filter_terms(int metric, float h, float c, float nrm, float qn, float gam, float rad,
                                              uint32_t id, float4 &tA, float2 &tC) {
-    const float sr = sqrtf(2.0f * h);
-    tC = make_float2(0.f, nrm);
-    if (metric == METRIC_ANGULAR) {
-        tA = make_float4(c + 0.5f * qn, sr, rad, __uint_as_float(id));
-        tC.x = 2.0f * (gam * sr * sqrtf(qn) + 0.5f * gam * qn + 2.4e-7f * (fabsf(c) + 0.5f * qn));
-    } else if (metric == METRIC_L2SQR) {   // everything halved (the radius exactly)
-        tA = make_float4(h - 6.0f * gam * h, sr, 0.5f * rad, __uint_as_float(id));
-    } else {
-        tA = make_float4(h - 2.0f * gam * h - 4.0f * gam * nrm, sr, rad, __uint_as_float(id));
-    }
+    const FilterRow r = filter_row((FilterMetric)metric, h, c, nrm, qn, gam, rad);
+    tA = make_float4(r.A, r.s, r.rad, __uint_as_float(id));
+    tC = make_float2(r.C, r.nrm);
 }
 
 // The tile's rows: entries [j0, j0 + nb) of U in rows 0 .. nb - 1, entries
@@ -496,26 +492,27 @@ __global__ void __launch_bounds__(TC_THREADS, JOIN_TC_MAX_CTAS_PER_SM)
                     unsigned need = uval ? (1u << cols) - 1u : 0u;
                     if (warp == 0 && (uint32_t)lane >= cb) need &= lane - cb >= 15 ? 0u : ~0u << (lane - cb + 1);
                     unsigned pm = 0;
+                    // the test of the pair with new entry j, the columns' entry c
+                    auto test = [&](uint32_t j, float gram, float &g, float &etp, float4 &ja) {
+                        ja = sh.tA[j];   // rows up to Umax: past j1 masked below
+                        g = gram;
+                        etp = et;
+                        float t2 = k2 * ja.y;
+                        if constexpr (PREC == 1) {   // the scales, and this pair's relative error
+                            const float2 jf = sh.tF[j];
+                            g = g * uf.x * jf.x;
+                            etp = filter_et8(uf.y, jf.y, g8);
+                            t2 = 2.f * etp * ua.y * ja.y;
+                        }
+                        const float2 jc = metric == METRIC_ANGULAR ? sh.tC[j] : make_float2(0.f, 0.f);
+                        return filter_pair((FilterMetric)metric, g, t2, gam, ua.x, ja.x, ua.z, ja.z, uc.x, jc.x, uc.y, jc.y);
+                    };
 #pragma unroll
                     for (int c = 0; c < 16; ++c) {
-                        const float4 ja = sh.tA[j0 + cb + c];   // rows up to Umax: past j1 masked below
-                        float g = v[c], t2 = k2 * ja.y;
-                        if constexpr (PREC == 1) {   // the scales, and this pair's relative error
-                            const float2 jf = sh.tF[j0 + cb + c];
-                            g = g * uf.x * jf.x;
-                            t2 = 2.f * (uf.y * jf.y * (1.f + g8) - 1.f) * ua.y * ja.y;
-                        }
-                        bool skip;
-                        if (metric == METRIC_ANGULAR) {
-                            const float2 jc = sh.tC[j0 + cb + c];
-                            const float full = g + (ua.x + ja.x), w = uc.y * jc.y;
-                            const float lhs = -full - t2 - (uc.x + jc.x) - 2.f * gam * w - 4.f * gam * fabsf(full) -
-                                              4.8e-7f * fabsf(g);
-                            skip = lhs > fmaxf(ua.z, ja.z) * (w + FLT_EPSILON);
-                        } else {
-                            skip = (ua.x + ja.x) - g - t2 > fmaxf(ua.z, ja.z);
-                        }
-                        if (!skip) pm |= 1u << c;
+                        float4 ja;
+                        float g, etp;
+                        const FilterTest ft = test(j0 + cb + c, v[c], g, etp, ja);
+                        if (!(ft.lhs > ft.rhs)) pm |= 1u << c;
                         const uint32_t idj = __float_as_uint(ja.w);
                         if (idj == NO_ID || (unew && idj == idu)) need &= ~(1u << c);
                     }
@@ -532,25 +529,29 @@ __global__ void __launch_bounds__(TC_THREADS, JOIN_TC_MAX_CTAS_PER_SM)
                         uint32_t at = 0;
                         if (lane == 31 && end) at = atomicAdd(jq.stail, end);
                         at = __shfl_sync(FULL, at, 31) + end - have;
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) {
+#pragma unroll 1   // (one copy: rarely run)
+                        for (int c = 0; c < (int)cols; ++c) {
                             const bool mine = (need >> c) & 1u;
                             if (!__any_sync(FULL, mine)) continue;
-                            const uint32_t j = j0 + cb + c;
-                            float g = v[c], etp = et;
-                            if constexpr (PREC == 1) {
-                                g = g * uf.x * sh.tF[j].x;
-                                etp = uf.y * sh.tF[j].y * (1.f + g8) - 1.f;
-                            }
-                            const uint4 e = make_uint4(n, idu, __float_as_uint(sh.tA[j].w), __float_as_uint(g));
-                            if (mine && at < JOIN_TC_SAMPLES) { jq.sample[at] = e; jq.setp[at] = etp; }
+                            float gram = 0.f;
+#pragma unroll
+                            for (int k = 0; k < 16; ++k)
+                                if (k == c) gram = v[k];
+                            float4 ja;
+                            float g, etp;
+                            const FilterTest ft = test(j0 + cb + c, gram, g, etp, ja);
+                            const uint4 e = make_uint4(n, idu, __float_as_uint(ja.w), __float_as_uint(g));
+                            const float4 f = make_float4(etp, ft.lhs, fmaxf(ua.z, ja.z), (pm >> c) & 1u ? 0.f : 1.f);
+                            if (mine && at < JOIN_TC_SAMPLES) { jq.sample[at] = e; jq.filter[at] = f; }
                             unsigned over = __ballot_sync(FULL, mine && at >= JOIN_TC_SAMPLES);
                             for (; over; over &= over - 1) {   // past the record's end: here
                                 const int src = __ffs(over) - 1;
                                 SampleTally t{};
                                 sample_pair(s, __shfl_sync(FULL, e.x, src), __shfl_sync(FULL, e.y, src),
                                             __shfl_sync(FULL, e.z, src), __uint_as_float(__shfl_sync(FULL, e.w, src)),
-                                            __shfl_sync(FULL, etp, src), lane, t);
+                                            make_float4(__shfl_sync(FULL, f.x, src), __shfl_sync(FULL, f.y, src),
+                                                        __shfl_sync(FULL, f.z, src), __shfl_sync(FULL, f.w, src)),
+                                            lane, t);
                                 if (lane == 0) t.add(s.tc);
                             }
                             at += mine;
@@ -621,7 +622,7 @@ __global__ void __launch_bounds__(256) join_sample_kernel(const __grid_constant_
     SampleTally t{};
     for (uint32_t e = blockIdx.x * 8 + (threadIdx.x >> 5); e < total; e += nw) {
         const uint4 p = jq.sample[e];
-        sample_pair(s, p.x, p.y, p.z, __uint_as_float(p.w), jq.setp[e], lane, t);
+        sample_pair(s, p.x, p.y, p.z, __uint_as_float(p.w), jq.filter[e], lane, t);
     }
     if (lane == 0 && t.sampled) t.add(s.tc);
 }
