@@ -697,9 +697,13 @@ size_t join_tc_smem(const BuildState &s, int prec) {
 
 }  // namespace
 
+// The rows and lists the join takes, else kg_build refuses: two tiles, a row and
+// 28 bytes per list entry within 200 KB.  (Of them every one fits the 227 KB of a
+// CTA as join_tc_smem lays it out: the longest lists go with the narrowest rows,
+// E4M3 rows of 32, 7,017 entries, 229,280 bytes.)
 bool join_tc_supported(const BuildState &s, int prec) {
-    // two CTAs an SM at least; wider rows take the CUDA-core join
-    return s.D.ld % (prec ? 32 : 16) == 0 && join_tc_smem(s, prec) + join_tc_tile(s, prec) <= 224 * 1024;
+    const size_t Umax = (size_t)s.NEWCAP + s.OLDCAP;
+    return s.D.ld % (prec ? 32 : 16) == 0 && 2 * join_tc_tile(s, prec) + (size_t)s.D.ld * 4 + Umax * 28 <= 200 * 1024;
 }
 
 uint64_t join_tc_node_max(const BuildState &s) {
