@@ -1574,24 +1574,6 @@ extern "C" int kg_build(kg_ctx *ctx, const kg_index_params *params, kg_index_inf
         return set_error(ctx, KG_E_INVALID, fp8 ? "tensor-core join (FP8): needs d padded to a multiple of 32 and "
                                                   "lists that fit in shared memory"
                                                 : "tensor-core join: lists do not fit in shared memory");
-    JoinQueue jq{};
-    uint64_t *jworst = nullptr, *jpre = nullptr, qcap = 0;
-    if (use_tc) {
-        // (x, y, node) entries for one round's pairs; rounds are cut to fit
-        qcap = std::max<uint64_t>(64ull << 20, 4 * join_tc_node_max(s));
-        if ((e = ctx->joinq.reserve(JOIN_TC_SAMPLES * 32ull + qcap * 12 + 64)) != cudaSuccess) return cuda_fail(ctx, e, "alloc join queue");
-        if ((e = ctx->joinaux.reserve((n + 1) * 16)) != cudaSuccess) return cuda_fail(ctx, e, "alloc join queue");
-        jq.sample = ctx->joinq.as<uint4>();
-        jq.filter = reinterpret_cast<float4 *>(jq.sample + JOIN_TC_SAMPLES);
-        jq.x = reinterpret_cast<uint32_t *>(jq.filter + JOIN_TC_SAMPLES);
-        jq.y = jq.x + qcap;
-        jq.n = jq.y + qcap;
-        jq.tail = reinterpret_cast<unsigned long long *>(jq.n + qcap + (qcap & 1));
-        jq.work = reinterpret_cast<uint32_t *>(jq.tail + 1);
-        jq.stail = jq.work + 1;
-        jworst = ctx->joinaux.as<uint64_t>();
-        jpre = jworst + n + 1;
-    }
     cudaMemsetAsync(s.rcnt_new + N, 0, 4, st);   // scan inputs carry one extra zero
     cudaMemsetAsync(s.rcnt_old + N, 0, 4, st);
 
@@ -1658,6 +1640,41 @@ extern "C" int kg_build(kg_ctx *ctx, const kg_index_params *params, kg_index_inf
         }
     }
     if (!s.off_lin) s.jt_rows = 0;   // locked inserts: the warp-per-node join
+
+    // The tensor-core join's queue of (x, y, node) entries for one round's pairs (rounds are cut to
+    // fit), its audit's record and the nodes' worst cases.  They lie in the grouped offers' buffer,
+    // which is written only after an iteration's last round; where that is too small (locked inserts,
+    // a bounded record) in a buffer of their own, given back after the build.
+    JoinQueue jq{};
+    uint64_t *jworst = nullptr, *jpre = nullptr, qcap = 0;
+    if (use_tc) {
+        const uint64_t node_max = join_tc_node_max(s), most = 64ull << 20;
+        const uint64_t least = std::max<uint64_t>(std::min<uint64_t>(most, n * 512), 4 * node_max);
+        qcap = std::max<uint64_t>(std::min<uint64_t>(most, n * 8192), 4 * node_max);
+        auto bytes = [&](uint64_t entries) { return JOIN_TC_SAMPLES * 32ull + entries * 12 + (n + 1) * 16 + 64; };
+        if (s.off_grp) {   // of a small data set up to 64 MB
+            if ((e = ctx->offer_grp.reserve(std::min<uint64_t>(bytes(qcap), 64 << 20))) != cudaSuccess)
+                return cuda_fail(ctx, e, "alloc join offers");
+            s.off_grp = ctx->offer_grp.as<uint4>();
+        }
+        const uint64_t have = s.off_grp ? ctx->offer_grp.bytes : 0;
+        if (have >= bytes(least)) {
+            qcap = std::min<uint64_t>(qcap, (have - bytes(0)) / 12);
+            jq.sample = ctx->offer_grp.as<uint4>();
+        } else {
+            if ((e = ctx->joinq.reserve(bytes(qcap))) != cudaSuccess) return cuda_fail(ctx, e, "alloc join queue");
+            jq.sample = ctx->joinq.as<uint4>();
+        }
+        jq.filter = reinterpret_cast<float4 *>(jq.sample + JOIN_TC_SAMPLES);
+        jq.x = reinterpret_cast<uint32_t *>(jq.filter + JOIN_TC_SAMPLES);
+        jq.y = jq.x + qcap;
+        jq.n = jq.y + qcap;
+        jq.tail = reinterpret_cast<unsigned long long *>(jq.n + qcap + (qcap & 1));
+        jq.work = reinterpret_cast<uint32_t *>(jq.tail + 1);
+        jq.stail = jq.work + 1;
+        jworst = reinterpret_cast<uint64_t *>(jq.tail + 2);
+        jpre = jworst + n + 1;
+    }
 
     // GenerateControl (kgraph.cpp:254-270): C distinct random nodes, exact K-NN.
     if (g_verbosity > 0) std::cerr << "Generating control..." << std::endl;
@@ -1927,6 +1944,8 @@ extern "C" int kg_build(kg_ctx *ctx, const kg_index_params *params, kg_index_inf
         return cuda_fail(ctx, e, "update graph");
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e, "update");
     ctx->last_build_graph_launches = graph_launches;
+
+    ctx->joinq.release();   // only needed while joining
 
     // finalize (kgraph.cpp:975-988) into the context's CSR graph
     DevBuf &cnt = ctx->build_scratch[22];

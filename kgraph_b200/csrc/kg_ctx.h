@@ -107,7 +107,7 @@ struct kg_ctx {
     kgb::DevBuf rev_scratch[15];     // reverse-edge completion work space (kg_graph.cu), kept between builds
     int join_mode = KG_JOIN_AUTO;
     kgb::DevBuf tcstat;              // tensor-core join counters
-    kgb::DevBuf joinq, joinaux, joinb;   // tensor-core join: candidate queue, worst-case prefix, round bounds
+    kgb::DevBuf joinq, joinb;        // tensor-core join: candidate queue (during a build), round bounds
     kgb::DevBuf offer_lin, offer_grp, offer_aux, offer_scan;   // deferred join inserts (kg_build.cu)
     int join_inserts = KG_INSERTS_AUTO;
     size_t offer_cap = 0;             // record-buffer capacity of deferred inserts, in offers (0: automatic)
