@@ -381,9 +381,10 @@ int kg_set_join_offer_capacity(kg_ctx *ctx, size_t offers);
  * candidate id, distance, source node with bit 31 set for a pair's x <- y
  * offer); found[source] is set to 1 where such an offer lands below K (other
  * entries 0).  A pool's offers are merged in ascending (distance, id) order in
- * passes of at most 256; `found` follows the serial inserts in the caller's
- * order of each pool's offers (their arrival order).  No counterpart in the
- * reference. */
+ * passes of at most 256 (the rest of a pool in the given order, once more than
+ * 512 offers cannot be told apart by a cut between distances); `found` follows
+ * the serial inserts in the caller's order of each pool's offers (their arrival
+ * order).  No counterpart in the reference. */
 int kg_join_merge_check(kg_ctx *ctx, unsigned n, unsigned L, unsigned K, float *pool_d, uint32_t *pool_i,
                         uint32_t *nodeL, float *radius, size_t n_off, const uint32_t *target, const uint32_t *cand,
                         const float *dist, const uint32_t *src, uint32_t *found);

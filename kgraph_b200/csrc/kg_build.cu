@@ -852,8 +852,58 @@ __device__ __forceinline__ void warp_sort_keys(unsigned long long *keys, int lan
 
 constexpr uint32_t MG_CH = 256;     // offers merged per pass at most (sorted in shared memory)
 constexpr uint32_t MG_PASS = 160;   // offers a value-mode pass aims at where they do not all fit
+constexpr uint32_t MG_TIES = 512;   // offers that no cut between distances separates and that still go in order
 constexpr int MG_WARPS = 8;
 size_t merge_warp_bytes(uint32_t PS) { return (size_t)MG_CH * 20 + (size_t)PS * 16; }
+
+// The next pass of a range [lo, hi] of (distance, id) keys that holds more than
+// MG_CH offers: its smallest, up to MG_CH of them, into keys.  A cut with too many
+// is narrowed by a sample of 32 of those it holds; copies of one offer beyond
+// MG_CH are counted in `more` only (they are duplicates).  Out of line: rarely run.
+struct TiePass { unsigned long long lo; uint32_t cm, more; };   // lo: the next pass's
+__device__ __noinline__ TiePass tie_pass(const uint4 *off, uint32_t m, unsigned long long lo, unsigned long long hi,
+                                         unsigned long long *keys, int lane) {
+    unsigned long long top = hi;   // a cut with too many
+    for (;;) {
+        uint32_t cm = 0;
+        for (uint32_t k0 = 0; k0 < m; k0 += 32) {
+            const uint32_t k = k0 + lane;
+            bool in = false;
+            unsigned long long key = 0;
+            if (k < m) {
+                const uint4 o = off[k];
+                key = (unsigned long long)f2ord(__uint_as_float(o.z)) << 32 | o.y;
+                in = key >= lo && key <= hi;
+            }
+            const unsigned bal = __ballot_sync(FULL, in);
+            const uint32_t pos = cm + __popc(bal & ((1u << lane) - 1u));
+            if (in && pos < MG_CH) keys[pos] = key;
+            cm += __popc(bal);
+        }
+        __syncwarp();
+        if (cm > MG_CH && hi > lo) {
+            top = hi;
+            unsigned long long sk = keys[lane * (MG_CH / 32)];
+            __syncwarp();
+#pragma unroll 1
+            for (int kk = 2; kk <= 32; kk <<= 1)   // sorted (bitonic across lanes)
+#pragma unroll 1
+                for (int jj = kk >> 1; jj > 0; jj >>= 1) {
+                    const unsigned long long other = __shfl_xor_sync(FULL, sk, jj);
+                    const bool keep_min = ((lane & jj) == 0) == ((lane & kk) == 0);
+                    if ((other < sk) == keep_min) sk = other;
+                }
+            hi = __shfl_sync(FULL, sk, (int)(MG_PASS * 32 / cm));
+            if (hi >= top) hi = __shfl_sync(FULL, sk, 0);
+            if (hi >= top) hi = top - 1;   // mostly copies of one offer
+        } else if (cm == 0 && hi < top) {   // all of them above this cut
+            lo = hi + 1;
+            hi = top;
+        } else {
+            return TiePass{hi + 1, min(cm, MG_CH), cm > MG_CH ? cm - MG_CH : 0u};
+        }
+    }
+}
 
 // Nhood::parallel_try_insert (kgraph.cpp:723-736) of every deferred offer
 // into its pool, one warp per pool, without locks (the join has finished).
@@ -980,14 +1030,17 @@ __global__ void __launch_bounds__(MG_WARPS * 32) offer_merge_kernel(BuildState s
         // distance key lies in (lo, hi], hi cut from a 32-offer sample so that
         // about MG_PASS fall in; passes follow in ascending order, so the pass
         // that meets the first radius rejection ends the pool (every later
-        // offer is farther).  A range that no sample cut keeps within MG_CH
-        // (massive ties) switches the rest of the pool to scan mode: chunks of
-        // up to MG_CH in record order, each merged as it comes.
+        // offer is as far or farther).  A range of up to MG_TIES that no sample
+        // cut keeps within MG_CH goes in passes cut between (distance, id) keys; a
+        // larger one (massive ties, or thousands of offers) switches the rest of
+        // the pool to scan mode: chunks of up to MG_CH in record order, each merged
+        // as it comes.
         uint32_t lo_key = 0, rem = m, cursor = 0;
-        bool have_lo = false, scan_mode = false, stop = false;
+        unsigned long long lo_tie = 0;   // within such a range, whose end is lo_key: where the next pass starts
+        bool have_lo = false, ties = false, scan_mode = false, stop = false;
         while (rem && !stop) {
-            uint32_t cm = 0;
-            if (!scan_mode) {
+            uint32_t cm = 0, more = 0;
+            if (!scan_mode && !ties) {
                 uint32_t hi_key = 0xFFFFFFFFu;
                 int idx = -1;
                 uint32_t sk = 0xFFFFFFFFu;
@@ -1006,7 +1059,7 @@ __global__ void __launch_bounds__(MG_WARPS * 32) offer_merge_kernel(BuildState s
                     if (nv == 0) scan_mode = true;
                     else idx = (int)min(nv - 1, (uint32_t)(((uint64_t)MG_PASS * nv) / rem));
                 }
-                while (!scan_mode) {
+                while (!scan_mode && !ties) {
                     if (idx >= 0) hi_key = __shfl_sync(FULL, sk, idx);
                     cm = 0;
                     for (uint32_t k0 = 0; k0 < m; k0 += 32) {
@@ -1029,8 +1082,16 @@ __global__ void __launch_bounds__(MG_WARPS * 32) offer_merge_kernel(BuildState s
                         have_lo = true;
                         break;
                     }
-                    if (idx <= 0) scan_mode = true;   // ties: no cut fits one pass
-                    else idx /= 2;
+                    if (idx > 0) {
+                        idx /= 2;
+                    } else if (cm <= MG_TIES) {
+                        ties = true;
+                        lo_tie = have_lo ? (unsigned long long)(lo_key + 1) << 32 : 0ull;   // (lo_key: not the last)
+                        lo_key = hi_key;
+                        have_lo = true;
+                    } else {
+                        scan_mode = true;
+                    }
                 }
                 __syncwarp();
             }
@@ -1055,8 +1116,19 @@ __global__ void __launch_bounds__(MG_WARPS * 32) offer_merge_kernel(BuildState s
                 }
                 __syncwarp();
             }
-            if (cm == 0) break;   // nothing left (the counts agree; this only guards the loop)
-            rem -= cm;
+            if (ties) {
+                const unsigned long long end = (unsigned long long)lo_key << 32 | 0xFFFFFFFFu;
+                const TiePass t = tie_pass(s.off_grp + o0, m, lo_tie, end, keys, lane);
+                cm = t.cm;
+                more = t.more;
+                lo_tie = t.lo;
+                ties = t.lo - 1 != end;
+            }
+            if (cm == 0) {
+                if (have_lo && !scan_mode && lo_key != 0xFFFFFFFFu) continue;   // a range's end: on with the next
+                break;   // nothing left (the counts agree; this only guards the loop)
+            }
+            rem -= cm + more;
             uint32_t P2 = 32;
             while (P2 < cm) P2 <<= 1;
             for (uint32_t k = cm + lane; k < P2; k += 32) keys[k] = ~0ull;
@@ -1153,11 +1225,11 @@ __global__ void __launch_bounds__(MG_WARPS * 32) offer_merge_kernel(BuildState s
                 }
             }
             ntail = __shfl_sync(FULL, ntail, 0);
-            // a radius rejection in value mode: the offers still to come are all farther
+            // a radius rejection in order: the offers still to come are all as far or farther
             stop = !scan_mode && __shfl_sync(FULL, rejected, 0);
             __syncwarp();
             // counts: offers that passed the radius test (duplicates included), and those that landed
-            att += (cm - nnd) + qs + ntail;
+            att += (cm - nnd) + more + qs + ntail;
             landed += qs + ntail;
             if (full_main || ntail) { rad = pdn[L - 1]; rad_set = true; }
             Lc = min(L, Lc + qs);
