@@ -181,7 +181,8 @@ KG_HD void gnu_sort(A &a, int first, int last) {
 //    left stop, or the last right stop swapped if that comes first.
 //  * The final insertion sort is stable, and ranges that were left have at most
 //    16 records: a record's place is its own plus the smaller ones up to 15
-//    behind it minus the larger ones up to 15 before it.
+//    behind it minus the larger ones up to 15 before it.  Among NaN a place
+//    is not a record's own any more: there one lane inserts.
 // A range whose depth limit is spent is heap-sorted by one lane.
 constexpr int WARP_SORT_MAX = 8191, WARP_SORT_TMP = 48;
 
@@ -272,6 +273,22 @@ __device__ inline void warp_gnu_sort(float *d, uint32_t *id, uint32_t *m, int n,
             __syncwarp();
         }
         f = cut;
+    }
+    bool nan = false;
+    for (int p = lane; p < n; p += 32) nan |= d[p] != d[p];
+    if (__any_sync(0xFFFFFFFFu, nan)) {
+        if (lane == 0) {
+            WarpSortAcc a{d, id, m};
+            gs_insertion_sort(a, 0, n < 16 ? n : 16);
+            for (int i = 16; i < n; ++i) {   // gs_unguarded_linear_insert, with a guard
+                const WarpSortAcc::Rec val = a.get(i);
+                int at = i;
+                for (; at > 0 && val.d < d[at - 1]; --at) a.put(at, a.get(at - 1));
+                a.put(at, val);
+            }
+        }
+        __syncwarp();
+        return;
     }
     // the final insertion sort; a piece of 32 is written once the next one has been ranked
     float pd = 0.f;
