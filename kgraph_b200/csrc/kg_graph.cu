@@ -86,14 +86,17 @@ __global__ void __launch_bounds__(REV_WARPS * 32) rev_assemble_kernel(uint32_t N
         float *ld = in_smem ? s_d[wib] : gd;
         // reverse edges from sources below x, then (behind the node's own) from sources above it
         uint32_t nb = 0;
+        bool nan = false;   // among the distances this lane stored
         for (uint32_t b = 0; b < rx; b += 32) {
             const uint32_t j = b + lane;
             const unsigned long long v = j < rx ? sval[q0 + j] : 0ull;
             const uint32_t src = (uint32_t)v;
             if (j < rx && src != x) {
                 const uint32_t at = src < x ? j : j + kx;
+                const float dd = __uint_as_float((uint32_t)(v >> 32));
                 li[at] = src;
-                ld[at] = __uint_as_float((uint32_t)(v >> 32));
+                ld[at] = dd;
+                nan |= dd != dd;
             }
             nb += __popc(__ballot_sync(ALL, j < rx && src < x));
         }
@@ -108,13 +111,14 @@ __global__ void __launch_bounds__(REV_WARPS * 32) rev_assemble_kernel(uint32_t N
                 const float dd = nbr_d[o0 + j];
                 li[at] = id;
                 ld[at] = dd;
+                nan |= dd != dd;
                 if ((self >> lane) & 1u) { li[at + 1] = x; ld[at + 1] = dd; }
             }
             ns += __popc(self);
         }
         __syncwarp();
         if (p <= (uint32_t)WARP_SORT_MAX) {
-            warp_gnu_sort(ld, li, nullptr, (int)p, s_tmp[wib], lane);   // kgraph.cpp:697
+            warp_gnu_sort(ld, li, nullptr, (int)p, s_tmp[wib], nan, lane);   // kgraph.cpp:697
         } else {
             if (lane == 0) { WarpSortAcc acc{ld, li, nullptr}; gnu_sort(acc, 0, (int)p); }
             __syncwarp();

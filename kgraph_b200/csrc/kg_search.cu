@@ -387,6 +387,7 @@ __global__ void __launch_bounds__(MB == 9 ? 128 : 256, MB) search_kernel(SearchA
             }
             __syncwarp();
             n_seed += L;
+            bool nan = false;   // a distance this lane stored
             // kgraph.cpp:468-475: mark, flag, distance, m = 0, M = actual_M
             for (uint32_t base = 0; base < L; base += 32) {
                 uint32_t j = base + lane;
@@ -406,12 +407,17 @@ __global__ void __launch_bounds__(MB == 9 ? 128 : 256, MB) search_kernel(SearchA
                 batch_dist<G>(a, s, qn, cnt, lane);
                 // an out-of-range starting point (the error is raised above) enters as id 0,
                 // unflagged: it is never expanded, so no adjacency row is read for it
-                if (j < L) { s.pd[j] = s.cd[lane]; s.pid[j] = bad ? 0u : (id | FLAG_BIT); }
+                if (j < L) {
+                    const float dd = s.cd[lane];
+                    nan |= dd != dd;
+                    s.pd[j] = dd;
+                    s.pid[j] = bad ? 0u : (id | FLAG_BIT);
+                }
                 __syncwarp();
             }
             // kgraph.cpp:476: std::sort by dist (GNU introsort order for ties)
             if (L <= (uint32_t)WARP_SORT_MAX) {
-                warp_gnu_sort(s.pd, s.pid, s.pm, (int)L, s.lid, lane);
+                warp_gnu_sort(s.pd, s.pid, s.pm, (int)L, s.lid, nan, lane);
             } else {
                 if (lane == 0) {
                     WarpSortAcc acc{s.pd, s.pid, s.pm};

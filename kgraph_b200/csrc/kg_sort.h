@@ -171,7 +171,8 @@ KG_HD void gnu_sort(A &a, int first, int last) {
 #ifdef __CUDACC__
 // gnu_sort of n <= WARP_SORT_MAX records (key d[i], payload id[i] and, unless
 // null, m[i]; shared or global memory) by one warp: the same permutation, ties
-// included.  tmp: WARP_SORT_TMP words of the warp's own shared memory.
+// included.  tmp: WARP_SORT_TMP words of the warp's own shared memory; nan:
+// whether a lane has met a NaN among the keys.
 //  * Which ranges are partitioned, and around which pivots, depends only on the
 //    data, and ranges are disjoint, so their order is free.
 //  * A Hoare partition swaps the t-th stop of its left scan (a record not below
@@ -242,7 +243,7 @@ __device__ inline int warp_partition(float *d, uint32_t *id, uint32_t *m, int f,
     }
 }
 
-__device__ inline void warp_gnu_sort(float *d, uint32_t *id, uint32_t *m, int n, uint32_t *tmp, int lane) {
+__device__ inline void warp_gnu_sort(float *d, uint32_t *id, uint32_t *m, int n, uint32_t *tmp, bool nan, int lane) {
     uint8_t *rank = reinterpret_cast<uint8_t *>(tmp + 32);   // 64 bytes behind 32 frames
     int sp = 0, f = 0, l = n, depth = n > 1 ? 2 * (31 - __clz(n)) : 0;
     for (;;) {
@@ -274,8 +275,6 @@ __device__ inline void warp_gnu_sort(float *d, uint32_t *id, uint32_t *m, int n,
         }
         f = cut;
     }
-    bool nan = false;
-    for (int p = lane; p < n; p += 32) nan |= d[p] != d[p];
     if (__any_sync(0xFFFFFFFFu, nan)) {
         if (lane == 0) {
             WarpSortAcc a{d, id, m};
