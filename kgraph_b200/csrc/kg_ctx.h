@@ -104,7 +104,7 @@ struct kg_ctx {
 
     kgb::DevBuf build_scratch[25];   // NN-descent state (kg_build.cu)
     kgb::HostBuf build_host;         // its statistics' landing place
-    kgb::DevBuf rev_scratch[15];     // reverse-edge completion work space (kg_graph.cu), kept between builds
+    kgb::DevBuf rev_scratch[14];     // reverse-edge completion work space (kg_graph.cu), kept between builds
     int join_mode = KG_JOIN_AUTO;
     kgb::DevBuf tcstat;              // tensor-core join counters
     kgb::DevBuf joinq, joinb;        // tensor-core join: candidate queue (during a build), round bounds

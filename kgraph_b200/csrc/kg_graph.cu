@@ -197,7 +197,7 @@ int graph_reverse(kg_ctx *ctx, int rev_k) {
     // time varied from build to build.  Buffers grow with 1/8 slack.
     DevBuf *R = ctx->rev_scratch;
     DevBuf &kcnt = R[0], &koff = R[1], &toff = R[2], &noff = R[3], &fdeg = R[4], &foff = R[5], &key = R[6], &val = R[7],
-           &skey = R[8], &sval = R[9], &tmp = R[10], &ai = R[11], &ad = R[12], &fi = R[13], &fd = R[14];
+           &skey = R[8], &sval = R[9], &tmp = R[10], &ad = R[11], &fi = R[12], &fd = R[13];
     auto grow = [](DevBuf &b, size_t bytes) { return b.reserve(bytes <= b.bytes ? bytes : bytes + bytes / 8); };
     auto fail = [&](const char *w) { return cuda_fail(ctx, e, w); };
     if ((e = grow(kcnt, (n + 1) * 8)) != cudaSuccess || (e = grow(koff, (n + 1) * 8)) != cudaSuccess ||
@@ -224,22 +224,21 @@ int graph_reverse(kg_ctx *ctx, int rev_k) {
     int end_bit = 1;
     while (end_bit < 32 && (1ull << end_bit) < n) ++end_bit;
     size_t tb = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, tb, key.as<uint32_t>(), skey.as<uint32_t>(), val.as<unsigned long long>(),
-                                    sval.as<unsigned long long>(), (int64_t)Ef, 0, end_bit, st);
+    cub::DoubleBuffer<uint32_t> keys(key.as<uint32_t>(), skey.as<uint32_t>());
+    cub::DoubleBuffer<unsigned long long> vals(val.as<unsigned long long>(), sval.as<unsigned long long>());
+    cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, vals, (int64_t)Ef, 0, end_bit, st);
     if ((e = grow(tmp, tb)) != cudaSuccess) return fail("alloc sort");
-    if ((e = cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.as<uint32_t>(), skey.as<uint32_t>(),
-                                             val.as<unsigned long long>(), sval.as<unsigned long long>(), (int64_t)Ef, 0,
-                                             end_bit, st)) != cudaSuccess)
+    if ((e = cub::DeviceRadixSort::SortPairs(tmp.p, tb, keys, vals, (int64_t)Ef, 0, end_bit, st)) != cudaSuccess)
         return fail("sort");
-    rev_offsets_kernel<<<grid * 2, 256, 0, st>>>(N, Ef, skey.as<uint32_t>(), toff.as<uint64_t>());
+    rev_offsets_kernel<<<grid * 2, 256, 0, st>>>(N, Ef, keys.Current(), toff.as<uint64_t>());
     rev_places_kernel<<<grid, 256, 0, st>>>(N, koff.as<uint64_t>(), toff.as<uint64_t>(), noff.as<uint64_t>());
     const uint64_t E2 = 2 * Ef;
-    if ((e = grow(ai, E2 * 4 + 4)) != cudaSuccess || (e = grow(ad, E2 * 4 + 4)) != cudaSuccess)
-        return fail("alloc reverse");
+    if ((e = grow(ad, E2 * 4 + 4)) != cudaSuccess) return fail("alloc reverse");
+    uint32_t *ai = reinterpret_cast<uint32_t *>(vals.Alternate());   // the assembled ids: room for 2 Ef of them
     std::cerr << "Reranking edges..." << std::endl;
     rev_assemble_kernel<<<ctx->num_sms * 6, REV_WARPS * 32, 0, st>>>(
         N, ctx->offsets.as<uint64_t>(), ctx->nbr.as<uint32_t>(), ctx->nbr_d.as<float>(), koff.as<uint64_t>(),
-        toff.as<uint64_t>(), sval.as<unsigned long long>(), ai.as<uint32_t>(), ad.as<float>(), fdeg.as<uint64_t>());
+        toff.as<uint64_t>(), vals.Current(), ai, ad.as<float>(), fdeg.as<uint64_t>());
     if ((e = cudaGetLastError()) != cudaSuccess) return fail("reverse");
     if ((e = scan_counts64(ctx, fdeg.as<uint64_t>(), foff.as<uint64_t>(), N)) != cudaSuccess) return fail("scan");
     uint64_t Efin = 0;
@@ -247,8 +246,8 @@ int graph_reverse(kg_ctx *ctx, int rev_k) {
     cudaStreamSynchronize(st);
     if ((e = grow(fi, Efin * 4 + 4)) != cudaSuccess || (e = grow(fd, Efin * 4 + 4)) != cudaSuccess)
         return fail("alloc reverse");
-    compact_kernel<<<grid * 2, 256, 0, st>>>(N, noff.as<uint64_t>(), foff.as<uint64_t>(), ai.as<uint32_t>(),
-                                             ad.as<float>(), fi.as<uint32_t>(), fd.as<float>(),
+    compact_kernel<<<grid * 2, 256, 0, st>>>(N, noff.as<uint64_t>(), foff.as<uint64_t>(), ai, ad.as<float>(),
+                                             fi.as<uint32_t>(), fd.as<float>(),
                                              ctx->Mnode.as<uint32_t>(), 1);
     if ((e = cudaGetLastError()) != cudaSuccess) return fail("reverse");
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return fail("reverse");
