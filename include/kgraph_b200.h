@@ -201,7 +201,7 @@ int kg_filter_bounds(kg_ctx *ctx, const float *queries, size_t nq, size_t q_stri
  *                         query, every row that can be among the K nearest, and
  *                         those are evaluated with the canonical FP32 distance.
  *                         No counterpart in the reference.  Memory: a BF16 copy
- *                         of the dataset (n * round_up(d, 16) * 2 bytes, and 32
+ *                         of the dataset (n * round_up(d, 16) * 2 bytes, and 16
  *                         bytes per row unless angular), built on first use, and
  *                         a work space that the number of rows does not grow:
  *                         queries are taken in batches of about half a gigabyte

@@ -129,9 +129,8 @@ __global__ void prep_rows_kernel(DataView D, const float *mu, uint64_t inv, __nv
                 const __nv_bfloat16 h0 = __float2bfloat16_rn(h);
                 const float r1 = h - __bfloat162float(h0);
                 const __nv_bfloat16 h1 = __float2bfloat16_rn(r1), h2 = __float2bfloat16_rn(r1 - __bfloat162float(h1));
-                Xe[2 * at] = make_uint4((uint32_t)__bfloat16_as_ushort(h0) | (uint32_t)__bfloat16_as_ushort(h1) << 16,
-                                        (uint32_t)__bfloat16_as_ushort(h2), 0u, 0u);
-                Xe[2 * at + 1] = make_uint4(0u, 0u, 0u, 0u);
+                Xe[at] = make_uint4((uint32_t)__bfloat16_as_ushort(h0) | (uint32_t)__bfloat16_as_ushort(h1) << 16,
+                                    (uint32_t)__bfloat16_as_ushort(h2), 0u, 0u);
             }
             m0 = fmax(m0, v2 < INFINITY ? sqrt(v2) : INFINITY);
             m1 = fmax(m1, e2 < INFINITY ? (double)e : INFINITY);
@@ -769,7 +768,7 @@ int bruteforce_prepare(kg_ctx *ctx) {
     }
     cudaError_t e;
     if ((e = ctx->bf_rows.reserve((size_t)n * ld * 2)) != cudaSuccess ||
-        (e = ctx->bf_meta.reserve(ctx->metric == METRIC_ANGULAR ? 0 : (size_t)n * 32)) != cudaSuccess ||
+        (e = ctx->bf_meta.reserve(ctx->metric == METRIC_ANGULAR ? 0 : (size_t)n * 16)) != cudaSuccess ||
         (e = ctx->bf_aux.reserve((size_t)ld * 12 + 64 + 64)) != cudaSuccess)
         return cuda_fail(ctx, e, "alloc brute-force rows");
     cudaStream_t st = ctx->stream;
@@ -897,7 +896,8 @@ static int bruteforce_batch(kg_ctx *ctx, const SweepPlan &p, const float *Q, uin
     if (!tc_bf16_map(&mQ, Qb, ld, nq, ld, 64, BF_Q) || !tc_bf16_map(&mX, ctx->bf_rows.p, ld, n, ld, 64, BF_R))
         return set_error(ctx, KG_E_CUDA, "brute force: tensor map");
     mE = mX;
-    if (ext && !tc_bf16_map(&mE, ctx->bf_meta.p, 16, n, 16, 16, BF_R, CU_TENSOR_MAP_SWIZZLE_32B))
+    // (rows of 8 in memory, 16 in the box: TMA fills the rest with zeros)
+    if (ext && !tc_bf16_map(&mE, ctx->bf_meta.p, 8, n, 8, 16, BF_R, CU_TENSOR_MAP_SWIZZLE_32B))
         return set_error(ctx, KG_E_CUDA, "brute force: tensor map");
     SweepArgs a{};
     a.ld = ld; a.nq = nq; a.nsub = nsub;
