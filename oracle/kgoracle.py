@@ -13,6 +13,7 @@ import ctypes as C
 import importlib.util
 import os
 import sys
+import unittest
 
 import numpy as np
 
@@ -226,11 +227,19 @@ def load_reference_module(isa=None):
     raise RuntimeError("reference module not built under %s" % d)
 
 
+class ReferenceMissing(unittest.SkipTest):
+    """The reference was not compiled here (its sources are not there): a test that needs it is
+    skipped at that point, what it checked before stands."""
+
+
 class RefLib:
     """The reference's C++ API (KGraph + MatrixOracle<l2sqr>) via oracle/ref_driver.cpp."""
 
     def __init__(self, isa=None):
-        self.lib = C.CDLL(os.path.join(reference_dir(isa), "libkgref.so"))
+        path = os.path.join(reference_dir(isa), "libkgref.so")
+        if not os.path.exists(path):
+            raise ReferenceMissing("reference not compiled here (%s)" % path)
+        self.lib = C.CDLL(path)
         u, f, i = C.c_uint, C.c_float, C.c_int
         self.lib.kgref_build_l2sqr.restype = i
         self.lib.kgref_build_l2sqr.argtypes = [_f32p, u, u, u, u, u, u, u, u, u, f, f, u, i,
