@@ -50,13 +50,10 @@ TARGET = 0.95
 # dram__bytes_write.sum) of this workload at full size (1M x 128, 10,000
 # queries, K=10), per launch: the plain walk at P=1000, the router-seeded walk
 # at P=5, and the local join (the shared-memory join, the offers' scatter and
-# the pools' merge) summed over the iterations of one warm build.  Captured
-# before the walk took candidates of several batches at a time and the join its
-# register tiles; on a 64-centre mixture of the same size the plain walk now moves
-# 135.3e9 and the join stage 450e9 over 15 iterations.
-SEARCH_DRAM_BYTES_PER_LAUNCH = 136.18e9
-ROUTER_SEARCH_DRAM_BYTES_PER_LAUNCH = 17.53e9
-BUILD_JOIN_DRAM_BYTES = 377.8e9
+# the pools' merge) summed over the iterations of one warm build.
+SEARCH_DRAM_BYTES_PER_LAUNCH = 136.94e9
+ROUTER_SEARCH_DRAM_BYTES_PER_LAUNCH = 19.16e9
+BUILD_JOIN_DRAM_BYTES = 362.9e9
 
 
 def _sample(c, n, rng, d):

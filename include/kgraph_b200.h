@@ -130,7 +130,9 @@ int kg_search_batch(kg_ctx *ctx, const float *queries, size_t nq, size_t q_strid
  *                    bits) - 1) S); elsewhere the 12-byte entry runs.
  *                    A new context starts with split 4, warps_per_block 0,
  *                    prefetch 2, regs 64, compact 1; until a shape is set or
- *                    tuned, a search on narrow rows takes split 2.
+ *                    tuned, kg_search_batch and kg_router_search take split 2
+ *                    on narrow rows (kg_last_search_shape tells;
+ *                    kg_search_batch_noalloc stays at 4).
  * ms / default_ms / variants are filled by kg_search_autotune. */
 typedef struct {
     unsigned split, warps_per_block, prefetch;
@@ -199,8 +201,10 @@ int kg_filter_bounds(kg_ctx *ctx, const float *queries, size_t nq, size_t q_stri
  *                         tcgen05 (FP32 accumulation) give an approximate
  *                         distance; a rigorous margin of its error selects, per
  *                         query, every row that can be among the K nearest, and
- *                         those are evaluated with the canonical FP32 distance.
- *                         No counterpart in the reference.  Memory: a BF16 copy
+ *                         those are evaluated with the canonical FP32 distance
+ *                         (data without a finite margin -- a NaN, an infinity,
+ *                         norms of 1e18 -- take the scan).  No counterpart in
+ *                         the reference.  Memory: a BF16 copy
  *                         of the dataset (n * round_up(d, 16) * 2 bytes, and 16
  *                         bytes per row unless angular), built on first use, and
  *                         a work space that the number of rows does not grow:
@@ -213,7 +217,8 @@ int kg_set_bruteforce_mode(kg_ctx *ctx, int mode);
  * that were scanned in full instead: those without a finite margin (a NaN, an
  * infinity or, angular, a zero norm in the query, or a data set whose rows are
  * all zero) and those whose margin admits more rows than a query has room for
- * (max(2048, 16 K), and half of that in one part of the rows). */
+ * (max(2048, 16 K) in all, twice an even share of that in any one part of the
+ * rows). */
 typedef struct {
     int tensor;
     unsigned long long candidates, full_scans;
@@ -365,7 +370,8 @@ int kg_set_join_precision(kg_ctx *ctx, int mode);
  *                        runs in rounds of consecutive nodes) are inserted under
  *                        the lock during the join;
  *   KG_INSERTS_AUTO      (default) KG_INSERTS_DEFERRED.
- * The tensor-core joins (KG_JOIN_BF16 / KG_JOIN_FP8 iterations) always lock. */
+ * The tensor-core joins (KG_JOIN_BF16 / KG_JOIN_FP8 iterations) hand the pairs
+ * that their filter leaves to the same inserts, with one merge an iteration. */
 enum { KG_INSERTS_AUTO = 0, KG_INSERTS_LOCKED = 1, KG_INSERTS_DEFERRED = 2 };
 int kg_set_join_inserts(kg_ctx *ctx, int mode);
 /* Bound on the deferred inserts' record buffers, in offers (32 bytes of device

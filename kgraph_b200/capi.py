@@ -395,7 +395,7 @@ class Context:
         return b.value, s.value
 
     def set_join_precision(self, mode):
-        """'auto' (BF16 tensor-core join for d >= 64), 'fp32', 'bf16' or 'bf16_always'."""
+        """'auto' (the FP32 join), 'fp32', 'bf16', 'bf16_always', 'fp8' or 'fp8_always'."""
         self._check(self.L.kg_set_join_precision(self.h, JOIN[mode] if isinstance(mode, str) else int(mode)))
 
     def join_merge_check(self, L, K, pool_d, pool_i, nodeL, radius, target, cand, dist, src):

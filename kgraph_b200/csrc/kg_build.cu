@@ -329,9 +329,9 @@ __device__ __forceinline__ void jt_acc(float4 &acc, const float4 &x, const float
     lane_acc(acc, x, y, L2 ? METRIC_L2SQR : METRIC_EUCLIDEAN);
 }
 
-// Canonical raw sums of the tile's pairs: pi[k] / pj[k] point at this lane's
-// part of rows k.  Returns in v[k] the pair (new entry 2 (t & 1) + (t >> 1),
-// partner k of this group).
+// Canonical raw sums of the tile's pairs from a 4-lane group's partial sums:
+// acc[i][j] are this lane's four of pair (new entry i, partner j).  Lane t ends
+// with new entry 2 (t & 1) + (t >> 1): v[k] is its pair with partner k.
 template <bool L2>
 __device__ __forceinline__ void jt_reduce(float4 (&acc)[4][4], int t, float (&v)[4]) {
     const bool o1 = t & 1, o2 = t & 2;

@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(256) join_sample_kernel(const __grid_constant_
 
 // Phase 2: the queued pairs, 8 per warp pass: canonical FP32 distance by
 // 4-lane groups, the unlocked radius pre-test of both endpoints, then the
-// locked inserts (Nhood::parallel_try_insert, kgraph.cpp:723-736) -- the
+// inserts, recorded or locked (Nhood::parallel_try_insert, kgraph.cpp:723-736) -- the
 // CUDA-core join's inner loop, at full occupancy.
 __global__ void __launch_bounds__(256) join_insert_kernel(BuildState s, JoinQueue jq) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
