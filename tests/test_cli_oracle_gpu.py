@@ -2,7 +2,7 @@
 
 test_formats_gpu.py holds them to the compiled reference; where that is not
 there, the oracle's search of the same index file (pinned to the reference,
-test_oracle_pin.py) is the judge.
+test_oracle_pin.py) decides.
 """
 import os
 import re
